@@ -1186,8 +1186,11 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
     }
     {
       StageScope sc(h, 1, st);
-      dim3 gf((L + FWD_CH - 1) / FWD_CH, (n + NPF * FWD_WARPS - 1) / (NPF * FWD_WARPS));
-      absorb_fwd_kernel<G, R, NPF><<<gf, 32 * FWD_WARPS, fwd_smem, st>>>(K, L, s.Lp, n, s.d_C, s.d_cmask,
+      constexpr int CH = fwd_channels<R>();
+      dim3 gf((L + CH - 1) / CH, (n + NPF * FWD_WARPS - 1) / (NPF * FWD_WARPS));
+      const int kper = fwd_layers_per_cta(K, (long long)gf.x * gf.y);
+      gf.z = (K + kper - 1) / kper;
+      absorb_fwd_kernel<G, R, NPF><<<gf, 32 * FWD_WARPS, fwd_smem, st>>>(K, kper, L, s.Lp, n, s.d_C, s.d_cmask,
                                                                    w.pv.Xg, w.OD);
       CK_LAUNCH(h);
       if (s.ov.n > 0) {   // the OPTRAN channels' water-vapour-line component

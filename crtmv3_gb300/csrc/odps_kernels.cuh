@@ -529,90 +529,133 @@ __global__ void __launch_bounds__(32) prep_kernel(SensorTables S, RefSums RS, Ba
 
 // ---------------------------------------------------------------------------
 // 2. absorption forward: OD[p][k][l] = sum_s C[k][s][l] * X[p][k][s].
-//    CTA = 32 channels (lanes) x FWD_WARPS warps, each warp NP profiles; the
-//    coefficient slice of each layer is staged in shared memory (double
-//    buffered, cp.async) and used by all warps.
+//    CTA = 32 * CPL channels x FWD_WARPS warps (NP profiles each) x kper
+//    layers; the coefficient slice of each layer is staged in shared memory
+//    (double buffered) and used by all warps.
+//
+//    Bound: the FP64 pipe (2 multiply-adds per clock and SM, 64 clocks per
+//    warp instruction and scheduler) in the FP64 form, shared-memory reads
+//    beside the FP32 pipe in the mixed one.  The layers are independent, so
+//    the grid's z axis splits them: with one CTA walking all 100 layers a
+//    single 22-channel profile took 1716 us on one scheduler (now 15 us), and
+//    250 x 616 channels ran as 160 CTAs on 152 SMs (two rounds, 5.2 ms; now
+//    2.5 ms, where the pipe's rate alone takes 2.4 ms).
+//    FP64: one channel per lane (32-channel sensors leave no half idle), the
+//    coefficients widened once per CTA on their way to shared memory by
+//    integer instructions (the conversion instruction shares the FP64 pipe),
+//    and a group's absent profiles cost nothing.
 // ---------------------------------------------------------------------------
 constexpr int FWD_WARPS = 4;
-constexpr int FWD_CH = 64;   // channels per CTA: 2 per lane
+// channels per lane: 2 in FP32 (halves the broadcast reads of X per multiply-add)
+template <class R> constexpr int fwd_cpl() { return sizeof(R) == 4 ? 2 : 1; }
+template <class R> constexpr int fwd_channels() { return 32 * fwd_cpl<R>(); }
 
-// Coefficient tile of one reference layer: NS slots x FWD_CH channels from l0.
-template <int NS>
-__device__ __forceinline__ void load_c_tile64(float (*dst)[FWD_CH], const float* __restrict__ C,
-                                              int k, int Lp, int l0, int tid, int nthreads) {
-  for (int i = tid; i < NS * (FWD_CH / 4); i += nthreads) {
-    const int s = i / (FWD_CH / 4), q = i % (FWD_CH / 4);
-    const int l = l0 + q * 4;
-    // rows are padded to a multiple of 32 channels; a half tile past the end reads zeros
-    cp_async16(&dst[s][q * 4], C + ((size_t)k * NS + s) * Lp + (l < Lp ? l : 0), l < Lp ? 16 : 0);
-  }
+// Layers per CTA: enough CTAs for some 24 per SM, so that the last round is
+// short beside the whole; never fewer than one layer.
+inline int fwd_layers_per_cta(int K, long long tiles) {
+  const long long want = 152LL * 24;
+  const long long z = tiles >= want ? 1 : (want + tiles - 1) / tiles;
+  return z >= K ? 1 : (int)((K + z - 1) / z);
 }
 
 template <int G, class R, int NP>
 constexpr size_t fwd_smem_bytes() {
-  return sizeof(float) * 2 * Group<G>::NS * FWD_CH + sizeof(R) * 2 * FWD_WARPS * Group<G>::NS * NP;
+  return sizeof(R) * 2 * Group<G>::NS * (fwd_channels<R>() + FWD_WARPS * NP);
 }
 
 template <int G, class R, int NP>
-__global__ void __launch_bounds__(32 * FWD_WARPS) absorb_fwd_kernel(int K, int L, int Lp, int n_chunk,
+__global__ void __launch_bounds__(32 * FWD_WARPS) absorb_fwd_kernel(int K, int kper, int L, int Lp, int n_chunk,
                                                                     const float* __restrict__ C,
                                                                     const unsigned* __restrict__ cmask,
                                                                     const R* __restrict__ Xg,
                                                                     R* __restrict__ OD) {
-  constexpr int NS = Group<G>::NS, J = Group<G>::J;
+  constexpr int NS = Group<G>::NS, J = Group<G>::J, CPL = fwd_cpl<R>(), CH = 32 * CPL;
   constexpr int XCH = NS * NP * (int)sizeof(R) / 16;   // 16-byte chunks of one warp's X slice
+  constexpr int NT = 32 * FWD_WARPS;
   extern __shared__ __align__(16) unsigned char fwd_smem[];
-  auto cs = reinterpret_cast<float (*)[NS][FWD_CH]>(fwd_smem);                       // [2][NS][FWD_CH]
-  auto xs = reinterpret_cast<R (*)[FWD_WARPS][NS * NP]>(fwd_smem + sizeof(float) * 2 * NS * FWD_CH);
+  auto cs = reinterpret_cast<R (*)[NS][CH]>(fwd_smem);                               // [2][NS][CH]
+  auto xs = reinterpret_cast<R (*)[FWD_WARPS][NS * NP]>(fwd_smem + sizeof(R) * 2 * NS * CH);
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int l0 = blockIdx.x * FWD_CH;
-  const int la = l0 + lane, lb = l0 + 32 + lane;
+  const int l0 = blockIdx.x * CH;
+  int lc[CPL];
+  unsigned mine = 0u;
+#pragma unroll
+  for (int c = 0; c < CPL; c++) {
+    lc[c] = l0 + 32 * c + lane;
+    if (lc[c] < L) mine |= cmask[lc[c]];
+  }
   const int pg = blockIdx.y * FWD_WARPS + wib;
   const int p0 = pg * NP;
-  const unsigned wmask = __reduce_or_sync(FULL, (la < L ? cmask[la] : 0u) | (lb < L ? cmask[lb] : 0u));
+  const unsigned wmask = __reduce_or_sync(FULL, mine);
   const R* Xb = Xg + (size_t)pg * K * NS * NP;
-  const bool group_ok = p0 < n_chunk;
+  const int live = min(NP, n_chunk - p0);   // profiles of this warp's group (<= 0: none)
+  const int k0 = blockIdx.z * kper, k1 = min(K, k0 + kper);
   auto stage = [&](int k, int buf) {
-    load_c_tile64<NS>(cs[buf], C, k, Lp, l0, threadIdx.x, 32 * FWD_WARPS);
-    if (group_ok) {
+    // rows are padded to a multiple of 32 channels; a half tile past the end reads zeros
+    for (int i = threadIdx.x; i < NS * (CH / 4); i += NT) {
+      const int s = i / (CH / 4), q = i % (CH / 4), l = l0 + q * 4;
+      const float* src = C + ((size_t)k * NS + s) * Lp + (l < Lp ? l : 0);
+      if constexpr (sizeof(R) == 4) {
+        cp_async16(&cs[buf][s][q * 4], src, l < Lp ? 16 : 0);
+      } else {
+        const float4 v = l < Lp ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        R* d = &cs[buf][s][q * 4];
+        d[0] = to_f64(v.x); d[1] = to_f64(v.y); d[2] = to_f64(v.z); d[3] = to_f64(v.w);
+      }
+    }
+    if (live > 0) {
       const R* src = Xb + (size_t)k * NS * NP;
       for (int i = lane; i < XCH; i += 32)
         cp_async16(&xs[buf][wib][i * (16 / sizeof(R))], src + i * (16 / sizeof(R)), 16);
     }
     cp_async_commit();
   };
-  stage(0, 0);
-  for (int k = 0; k < K; k++) {
-    cp_async_wait_all();
-    __syncthreads();
-    if (k + 1 < K) stage(k + 1, (k + 1) & 1);
-    if (!group_ok) continue;
-    const float (*ct)[FWD_CH] = cs[k & 1];
-    const R* xk = xs[k & 1][wib];
-    R acc0[NP], acc1[NP];
+  // N of the group's profiles from pb on, all channels of the lane
+  auto layer = [&](auto nc, int k, int pb) {
+    constexpr int N = decltype(nc)::value;
+    const R (*ct)[CH] = cs[k & 1];
+    const R* xk = xs[k & 1][wib] + pb;
+    R acc[CPL][N];
 #pragma unroll
-    for (int p = 0; p < NP; p++) acc0[p] = acc1[p] = R(0);
+    for (int c = 0; c < CPL; c++)
+#pragma unroll
+      for (int p = 0; p < N; p++) acc[c][p] = R(0);
     static_for<J>([&](auto jc) {
       constexpr int j = decltype(jc)::value;
       constexpr int s0 = Group<G>::OFF[j], s1 = Group<G>::OFF[j + 1];
       if (!(wmask & (1u << j))) return;
 #pragma unroll
       for (int s = s0; s < s1; s++) {
-        const R ca = R(ct[s][lane]), cb = R(ct[s][32 + lane]);
-        R x[NP];
+        R x[N];
 #pragma unroll
-        for (int p = 0; p < NP; p++) x[p] = xk[s * NP + p];
+        for (int p = 0; p < N; p++) x[p] = xk[s * NP + p];
 #pragma unroll
-        for (int p = 0; p < NP; p++) { acc0[p] += ca * x[p]; acc1[p] += cb * x[p]; }
+        for (int c = 0; c < CPL; c++) {
+          const R cv = ct[s][32 * c + lane];
+#pragma unroll
+          for (int p = 0; p < N; p++) acc[c][p] += cv * x[p];
+        }
       }
     });
 #pragma unroll
-    for (int p = 0; p < NP; p++) {
-      if (p0 + p >= n_chunk) break;
-      R* o = OD + ((size_t)(p0 + p) * K + k) * L;
-      if (la < L) o[la] = acc0[p];
-      if (lb < L) o[lb] = acc1[p];
+    for (int p = 0; p < N; p++) {
+      if (p0 + pb + p >= n_chunk) break;
+      R* o = OD + ((size_t)(p0 + pb + p) * K + k) * L;
+#pragma unroll
+      for (int c = 0; c < CPL; c++)
+        if (lc[c] < L) o[lc[c]] = acc[c][p];
     }
+  };
+  stage(k0, k0 & 1);
+  for (int k = k0; k < k1; k++) {
+    cp_async_wait_all();
+    __syncthreads();
+    if (k + 1 < k1) stage(k + 1, (k + 1) & 1);
+    if (live <= 0) continue;
+    if (sizeof(R) == 4 || live == NP)
+      layer(std::integral_constant<int, NP>{}, k, 0);
+    else
+      for (int pb = 0; pb < live; pb++) layer(std::integral_constant<int, 1>{}, k, pb);
   }
 }
 
