@@ -1157,7 +1157,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
   BatchView bv = make_view(b);
   bv.perm = perm;
   constexpr int NPF = Tune<G, R>::FWD, NPA = Tune<G, R>::AD;
-  const size_t prep_smem = prep_smem_bytes<G>(K);
+  const size_t prep_smem = prep_smem_bytes<G>(K, Kmax);
   const size_t col_smem = column_smem_bytes<R>(K, Kmax);
   // channels per map CTA: 16 (more resident CTAs hide the tile loads; C2:
   // 6.4 ms against 7.4 ms with 32 and 8.1 ms with 8), fewer if the tiles exceed
@@ -1181,7 +1181,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
     const int n = std::min(chunk, P - p0);
     {
       StageScope sc(h, 0, st);
-      prep_kernel<G, R><<<n, 32, prep_smem, st>>>(s.tables, s.refsums, bv, w.pv, w.idx_map, p0, n);
+      prep_kernel<G, R><<<n, PREP_THREADS, prep_smem, st>>>(s.tables, s.refsums, bv, w.pv, w.idx_map, p0, n);
       CK_LAUNCH(h);
     }
     {

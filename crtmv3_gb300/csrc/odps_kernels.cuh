@@ -1,7 +1,7 @@
 // CUDA kernels of the clear-sky ODPS + Emission forward / K-matrix / adjoint path.
 //
 // A batch is processed in chunks of profiles.  Per chunk:
-//   prep_kernel        one warp per profile: Map_Input (ODPS_CoordinateMapping.f90:151-319),
+//   prep_kernel        one CTA per profile: Map_Input (ODPS_CoordinateMapping.f90:151-319),
 //                      running sums by warp scans, predictors X
 //                      (ODPS_Predictor.f90:645-1095) and the predictor
 //                      partial-derivative table D; mapping bands for the adjoint
@@ -279,29 +279,42 @@ struct PrepView {
   int K, Kmax, npf, npa;
 };
 
+constexpr int PREP_THREADS = 128;
+
 template <int G>
-inline size_t prep_smem_bytes(int K) {
+inline size_t prep_smem_bytes(int K, int Kmax) {
   return sizeof(double) * ((size_t)(4 + 3 * Group<G>::JM) * K + 2 * MAX_LAYERS + 1) +
-         sizeof(int) * (size_t)K;
+         sizeof(int) * (5 * (size_t)K + 2 + 2 * ((size_t)Kmax + 1) + 2 * (size_t)Kmax);
 }
 
 // ---------------------------------------------------------------------------
-// 1. prep: one warp (= one CTA) per profile
+// 1. prep: one CTA of 4 warps per profile, threads over the layers and levels.
+//
+//    Bound: FP64 issue (Map_Input, the running sums and, in the FP64 form, the
+//    predictors) and the latency of its chain; the bytes are small.  One warp
+//    per profile kept three of an SM's four schedulers idle and found the
+//    level brackets on one lane: 253 us for a single profile (FP64 form, 22
+//    channels; now 55 us).  With a thread
+//    per layer and level the brackets come from bisection (user levels are
+//    ascending; other orders take the sequential search, same result) and the
+//    transposed bands from shared-memory minima and maxima.
 // ---------------------------------------------------------------------------
 template <int G, class R>
-__global__ void __launch_bounds__(32) prep_kernel(SensorTables S, RefSums RS, BatchView b,
-                                                  PrepView<R> pv, const int* __restrict__ idx_map,
-                                                  int p_begin, int n_chunk) {
+__global__ void __launch_bounds__(PREP_THREADS) prep_kernel(SensorTables S, RefSums RS, BatchView b,
+                                                            PrepView<R> pv, const int* __restrict__ idx_map,
+                                                            int p_begin, int n_chunk) {
   constexpr int JM = Group<G>::JM, NS = Group<G>::NS, NNZ = DLayout<G>::NNZ, NX = DLayout<G>::NX;
   extern __shared__ double psm[];
-  const int lane = threadIdx.x;
+  __shared__ struct { double sv, zoff, sec_surface, cos_sensor; } geo;
+  __shared__ int sstatus, ascending;
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
   const int p = blockIdx.x;
   if (p >= n_chunk) return;
   const int gp = batch_profile(b, p_begin + p);
   const int K = S.K, Kmax = pv.Kmax;
   const int Ku = b.n_layers[gp];
   if (Ku < 2 || Ku > Kmax || Ku > MAX_LAYERS) {
-    if (lane == 0) pv.status[p] = ST_BAD_LAYERS;
+    if (tid == 0) pv.status[p] = ST_BAD_LAYERS;
     return;
   }
   double* sT = psm;                      // [K]     mapped temperature
@@ -313,25 +326,65 @@ __global__ void __launch_bounds__(32) prep_kernel(SensorTables S, RefSums RS, Ba
   double* ulnp = sGt + (size_t)JM * K;   // [MAX_LAYERS]
   double* ulev = ulnp + MAX_LAYERS;      // [MAX_LAYERS+1]
   int* sPass = reinterpret_cast<int*>(ulev + MAX_LAYERS + 1);  // [K]
+  int* sI0 = sPass + K;                  // [K]   band of each reference layer
+  int* sN = sI0 + K;                     // [K]
+  int* sLo = sN + K;                     // [K+1] user levels whose bracket touches a reference level
+  int* sHi = sLo + K + 1;                // [K+1]
+  int* sK1 = sHi + K + 1;                // [Kmax+1] brackets of the user levels
+  int* sK2 = sK1 + Kmax + 1;             // [Kmax+1]
+  int* sB0 = sK2 + Kmax + 1;             // [Kmax] reference layers mapping to a user layer
+  int* sB1 = sB0 + Kmax;                 // [Kmax]
   const double* lev = b.level_pressure + (size_t)gp * (Kmax + 1);
   const double* lay = b.pressure + (size_t)gp * Kmax;
   const double* tu = b.temperature + (size_t)gp * Kmax;
-  for (int k = lane; k < Ku; k += 32) ulnp[k] = log(lay[k]);
-  for (int k = lane; k <= Ku; k += 32)
+  for (int k = tid; k < Ku; k += PREP_THREADS) {
+    ulnp[k] = log(lay[k]);
+    sB0[k] = K;
+    sB1[k] = -1;
+  }
+  for (int k = tid; k <= Ku; k += PREP_THREADS)
     ulev[k] = (k == 0) ? ((lev[0] <= 0.0) ? log(lev[1] / 2.0) : log(lev[0])) : log(lev[k]);
-  __syncwarp();
-  int status = ST_OK;
+  for (int k = tid; k <= K; k += PREP_THREADS) { sLo[k] = Ku + 1; sHi[k] = -1; }
+  if (tid == 0) { sstatus = ST_OK; ascending = 1; }
+  __syncthreads();
+  // ---- height-dependent secants (ODPS_CoordinateMapping.f90:285-306), on
+  // the warp with the fewest layers
+  if (tid == PREP_THREADS - 1) {
+    const Geom g = geometry(b.zenith[gp]);
+    const double alt = b.altitude ? b.altitude[gp] : 0.0;
+    const double psfc = lev[Ku];
+    int sfc_idx = K;
+    double sfc_frac = 0.0;
+    if (S.ref_lev[K] > psfc) {
+      for (int k = K; k >= 0; k--)
+        if (S.ref_lev[k] < psfc) {
+          sfc_idx = k + 1;
+          sfc_frac = (S.ref_lev_lnp[sfc_idx] - ulev[Ku]) / (S.ref_lev_lnp[sfc_idx] - S.ref_lev_lnp[k]);
+          break;
+        }
+    }
+    double zoff;
+    if (S.ref_lev[K] >= psfc)
+      zoff = -(S.zgeo[sfc_idx] + sfc_frac * (S.zgeo[sfc_idx - 1] - S.zgeo[sfc_idx])) + alt;
+    else
+      zoff = CC_H * S.ref_t[K - 1] * log(1013.0 / S.ref_lev[K]);
+    geo.sv = (EARTH_RADIUS + alt) * sin(g.trans_zenith_radian);
+    geo.zoff = zoff;
+    geo.sec_surface = g.sec_trans_zenith;
+    geo.cos_sensor = 1.0 / g.sec_sensor_zenith;  // Common_RTSolution.f90:227
+  }
   int* bi0 = pv.band_i0 + (size_t)p * K;
   int* bn = pv.band_n + (size_t)p * K;
   double* bw = pv.band_w + (size_t)p * K * MAX_BAND;
-  // ---- mapping of T and absorbers to the reference layers (lanes stride over layers)
-  for (int k = lane; k < K; k += 32) {
+  // ---- mapping of T and absorbers to the reference layers
+  for (int k = tid; k < K; k += PREP_THREADS) {
     const int st = layer_avg_start(S.ref_lnp, K, ulnp, Ku, k);
     int i0, n;
     double* w = bw + (size_t)k * MAX_BAND;
-    status |= layer_avg_column(S.ref_lnp, K, ulnp, Ku, k, st, &i0, &n, w);
-    bi0[k] = i0;
-    bn[k] = n;
+    const int bad = layer_avg_column(S.ref_lnp, K, ulnp, Ku, k, st, &i0, &n, w);
+    if (bad) atomicOr(&sstatus, bad);
+    bi0[k] = sI0[k] = i0;
+    bn[k] = sN[k] = n;
     double acc = 0.0;
     for (int i = 0; i < n; i++) acc += w[i] * tu[i0 + i];
     sT[k] = acc;
@@ -354,12 +407,19 @@ __global__ void __launch_bounds__(32) prep_kernel(SensorTables S, RefSums RS, Ba
       sA[a * K + k] = v;
     }
     sPass[k] = pass;
+    for (int i = 0; i < n; i++) {
+      const int ku = i0 + i;
+      if (ku < Ku) { atomicMin(&sB0[ku], k); atomicMax(&sB1[ku], k); }
+    }
   }
-  __syncwarp();
-  // ---- running sums: contiguous block per lane, warp scan of the block totals
+  for (int i = tid; i < Ku; i += PREP_THREADS)
+    if (!(ulev[i] <= ulev[i + 1])) ascending = 0;
+  __syncthreads();
+  // ---- running sums, one warp per sum: a contiguous block of layers per
+  // lane, warp scan of the block totals
   {
     const int per = (K + 31) / 32, k0 = min(K, lane * per), k1 = min(K, k0 + per);
-    for (int qn = 0; qn < 2 + 2 * JM; qn++) {
+    for (int qn = wib; qn < 2 + 2 * JM; qn += PREP_THREADS / 32) {
       // qn: 0 T, 1 pdp*T, 2+a pdp*A_a, 2+JM+a pdp*A_a*T
       const int a = (qn < 2) ? 0 : (qn - 2) % JM;
       double* out = qn == 0 ? sTz : (qn == 1 ? sTzp : (qn < 2 + JM ? sGz + a * K : sGt + a * K));
@@ -378,34 +438,94 @@ __global__ void __launch_bounds__(32) prep_kernel(SensorTables S, RefSums RS, Ba
       }
     }
   }
-  __syncwarp();
-  // ---- height-dependent secants (ODPS_CoordinateMapping.f90:285-306)
-  const Geom g = geometry(b.zenith[gp]);
-  const double alt = b.altitude ? b.altitude[gp] : 0.0;
-  const double psfc = lev[Ku];
-  int sfc_idx = K;
-  double sfc_frac = 0.0;
-  if (S.ref_lev[K] > psfc) {
-    for (int k = K; k >= 0; k--)
-      if (S.ref_lev[k] < psfc) {
-        sfc_idx = k + 1;
-        sfc_frac = (S.ref_lev_lnp[sfc_idx] - ulev[Ku]) / (S.ref_lev_lnp[sfc_idx] - S.ref_lev_lnp[k]);
-        break;
+  // ---- reference -> user level brackets (Compute_Interp_Index): the first
+  // reference interval that holds the level, (0, 0) above the top level and
+  // (K, K) below the bottom one
+  {
+    const double* x = S.ref_lev_lnp;
+    if (ascending) {
+      for (int i = tid; i <= Ku; i += PREP_THREADS) {
+        const double u = ulev[i];
+        int a = 0, c = 0;
+        if (u > x[K]) {
+          a = c = K;
+        } else if (!(u < x[0])) {
+          int lo = 1, hi = K;   // first ix with u <= x[ix]
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (u <= x[mid]) hi = mid; else lo = mid + 1;
+          }
+          a = lo - 1; c = lo;
+        }
+        sK1[i] = a;
+        sK2[i] = c;
       }
+    } else if (tid == 0) {
+      const int nx = K + 1, nu = Ku + 1;
+      for (int i = 0; i < nu; i++) { sK1[i] = 0; sK2[i] = 0; }   // every entry a valid level
+      int k1 = nu + 1, k2 = 0;
+      for (int iu = 1; iu <= nu; iu++) {
+        if (ulev[iu - 1] < x[0]) { sK1[iu - 1] = 0; sK2[iu - 1] = 0; }
+        else { k1 = iu; break; }
+      }
+      for (int iu = nu; iu >= k1; iu--) {
+        if (ulev[iu - 1] > x[nx - 1]) { sK1[iu - 1] = nx - 1; sK2[iu - 1] = nx - 1; }
+        else { k2 = iu; break; }
+      }
+      int jj = 1;
+      for (int iu = k1; iu <= k2; iu++)
+        for (int ix = jj; ix <= nx - 1; ix++)
+          if (ulev[iu - 1] >= x[ix - 1] && ulev[iu - 1] <= x[ix]) {
+            sK1[iu - 1] = ix - 1; sK2[iu - 1] = ix; jj = ix;
+            break;
+          }
+    }
   }
-  double zoff;
-  if (S.ref_lev[K] >= psfc)
-    zoff = -(S.zgeo[sfc_idx] + sfc_frac * (S.zgeo[sfc_idx - 1] - S.zgeo[sfc_idx])) + alt;
-  else
-    zoff = CC_H * S.ref_t[K - 1] * log(1013.0 / S.ref_lev[K]);
-  const double sv = (EARTH_RADIUS + alt) * sin(g.trans_zenith_radian);
-  // ---- predictors and partials (lanes stride over layers)
+  __syncthreads();
+  {
+    int* k1o = pv.ulev_k1 + (size_t)p * (Kmax + 1);
+    int* k2o = pv.ulev_k2 + (size_t)p * (Kmax + 1);
+    double* fo = pv.ulev_fac + (size_t)p * (Kmax + 1);
+    const double* x = S.ref_lev_lnp;
+    for (int i = tid; i <= Ku; i += PREP_THREADS) {
+      const int a = sK1[i], c = sK2[i];
+      k1o[i] = a;
+      k2o[i] = c;
+      fo[i] = (a == c) ? 0.0 : (ulev[i] - x[a]) / (x[c] - x[a]);
+      // reference level <- user levels whose bracket touches it (path adjoint)
+      atomicMin(&sLo[a], i); atomicMax(&sHi[a], i);
+      atomicMin(&sLo[c], i); atomicMax(&sHi[c], i);
+    }
+    if (tid == 0) {
+      pv.scal[(size_t)p * 4 + 0] = geo.sec_surface;
+      pv.scal[(size_t)p * 4 + 1] = geo.cos_sensor;
+    }
+  }
+  // ---- user layer ku <- reference layers mapping to it (Map_Input adjoint)
+  {
+    int* uk0 = pv.ub_k0 + (size_t)p * Kmax;
+    int* un = pv.ub_n + (size_t)p * Kmax;
+    double* uw = pv.ub_w + (size_t)p * Kmax * MAX_UBAND;
+    for (int ku = tid; ku < Ku; ku += PREP_THREADS) {
+      const int k0 = sB0[ku], k1 = sB1[ku];
+      int n = (k1 < 0) ? 0 : k1 - k0 + 1;
+      if (n > MAX_UBAND) { atomicOr(&sstatus, (int)ST_UBAND_OVERFLOW); n = MAX_UBAND; }
+      uk0[ku] = k1 < 0 ? 0 : k0;
+      un[ku] = n;
+      if (pv.Dg)   // the weights: K-matrix and adjoint only
+        for (int i = 0; i < n; i++) {
+          const int k = k0 + i, r = ku - sI0[k];
+          uw[(size_t)ku * MAX_UBAND + i] = (r >= 0 && r < sN[k]) ? bw[(size_t)k * MAX_BAND + r] : 0.0;
+        }
+    }
+  }
+  // ---- predictors and partials (threads stride over layers)
   const int pgf = p / pv.npf, pof = p % pv.npf;
   const int pga = pv.npa ? p / pv.npa : 0, poa = pv.npa ? p % pv.npa : 0;
-  for (int k = lane; k < K; k += 32) {
+  for (int k = tid; k < K; k += PREP_THREADS) {
     // the predictors and partials are evaluated in R: FP32 in the mixed form
     LayerStateT<R> Ls;
-    const double sa = sv / (EARTH_RADIUS + (S.zgeo[k + 1] + zoff));
+    const double sa = geo.sv / (EARTH_RADIUS + (S.zgeo[k + 1] + geo.zoff));
     Ls.sec = R(1.0 / sqrt(1.0 - sa * sa));
     Ls.T_ = R(sT[k]);
     Ls.Tref = R(S.ref_t[k]);
@@ -446,85 +566,23 @@ __global__ void __launch_bounds__(32) prep_kernel(SensorTables S, RefSums RS, Ba
     }
   }
   // ---- compact-OPTRAN predictors (ODPS_Predictor.f90:336-347): a running
-  // sum over the layers, on lane 0, in FP64
+  // sum over the layers, on one thread, in FP64
   if (pv.opt) {
-    __syncwarp();
-    if (lane == 0) {
+    if (tid == 0) {
       double secl[MAX_LAYERS];
       for (int k = 0; k < K; k++) {
-        const double sa = sv / (EARTH_RADIUS + (S.zgeo[k + 1] + zoff));
+        const double sa = geo.sv / (EARTH_RADIUS + (S.zgeo[k + 1] + geo.zoff));
         secl[k] = 1.0 / sqrt(1.0 - sa * sa);
       }
       optran_profile(K, sT, sA + (size_t)S.h2o_idx * K, secl, sPass, S.ref_lev, S.ref_p, S.o_alpha, S.o_c1,
                      S.o_c2, pv.opt + (size_t)p * K * OPT_NS);
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) status |= __shfl_xor_sync(FULL, status, o);
-  // ---- reference -> user level brackets (Compute_Interp_Index, sequential on lane 0)
-  int* k1o = pv.ulev_k1 + (size_t)p * (Kmax + 1);
-  int* k2o = pv.ulev_k2 + (size_t)p * (Kmax + 1);
-  double* fo = pv.ulev_fac + (size_t)p * (Kmax + 1);
-  for (int i = lane; i <= Ku; i += 32) { k1o[i] = 0; k2o[i] = 0; }   // every entry a valid level
-  __syncwarp();
-  if (lane == 0) {
-    const double* x = S.ref_lev_lnp;
-    const int nx = K + 1, nu = Ku + 1;
-    int k1 = nu + 1, k2 = 0;
-    for (int iu = 1; iu <= nu; iu++) {
-      if (ulev[iu - 1] < x[0]) { k1o[iu - 1] = 0; k2o[iu - 1] = 0; }
-      else { k1 = iu; break; }
-    }
-    for (int iu = nu; iu >= k1; iu--) {
-      if (ulev[iu - 1] > x[nx - 1]) { k1o[iu - 1] = nx - 1; k2o[iu - 1] = nx - 1; }
-      else { k2 = iu; break; }
-    }
-    int jj = 1;
-    for (int iu = k1; iu <= k2; iu++)
-      for (int ix = jj; ix <= nx - 1; ix++)
-        if (ulev[iu - 1] >= x[ix - 1] && ulev[iu - 1] <= x[ix]) {
-          k1o[iu - 1] = ix - 1; k2o[iu - 1] = ix; jj = ix;
-          break;
-        }
-    for (int i = 0; i < nu; i++) {
-      const int a = k1o[i], c = k2o[i];
-      fo[i] = (a == c) ? 0.0 : (ulev[i] - x[a]) / (x[c] - x[a]);
-    }
-    pv.scal[(size_t)p * 4 + 0] = g.sec_trans_zenith;
-    pv.scal[(size_t)p * 4 + 1] = 1.0 / g.sec_sensor_zenith;  // Common_RTSolution.f90:227
-  }
-  __syncwarp();
-  // ---- reference level j <- user levels whose bracket touches it (path adjoint)
+  __syncthreads();
   int* ilo = pv.rlev_ilo + (size_t)p * (K + 1);
   int* ihi = pv.rlev_ihi + (size_t)p * (K + 1);
-  for (int jl = lane; jl <= K; jl += 32) {
-    int lo = Ku + 1, hi = -1;
-    for (int i = 0; i <= Ku; i++)
-      if (k1o[i] == jl || k2o[i] == jl) { if (i < lo) lo = i; hi = i; }
-    ilo[jl] = lo;
-    ihi[jl] = hi;
-  }
-  // ---- user layer ku <- reference layers mapping to it (Map_Input adjoint)
-  int* uk0 = pv.ub_k0 + (size_t)p * Kmax;
-  int* un = pv.ub_n + (size_t)p * Kmax;
-  double* uw = pv.ub_w + (size_t)p * Kmax * MAX_UBAND;
-  int ust = 0;
-  for (int ku = lane; ku < Ku; ku += 32) {
-    int k0 = -1, k1 = -1;
-    for (int k = 0; k < K; k++)
-      if (ku >= bi0[k] && ku < bi0[k] + bn[k]) { if (k0 < 0) k0 = k; k1 = k; }
-    int n = (k0 < 0) ? 0 : k1 - k0 + 1;
-    if (n > MAX_UBAND) { ust |= ST_UBAND_OVERFLOW; n = MAX_UBAND; }
-    uk0[ku] = k0 < 0 ? 0 : k0;
-    un[ku] = n;
-    for (int i = 0; i < n; i++) {
-      const int k = k0 + i, r = ku - bi0[k];
-      uw[(size_t)ku * MAX_UBAND + i] = (r >= 0 && r < bn[k]) ? bw[(size_t)k * MAX_BAND + r] : 0.0;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ust |= __shfl_xor_sync(FULL, ust, o);
-  if (lane == 0) pv.status[p] = status | ust;
+  for (int jl = tid; jl <= K; jl += PREP_THREADS) { ilo[jl] = sLo[jl]; ihi[jl] = sHi[jl]; }
+  if (tid == 0) pv.status[p] = sstatus;
 }
 
 // ---------------------------------------------------------------------------
