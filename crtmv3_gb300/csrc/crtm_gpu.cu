@@ -808,7 +808,8 @@ template <class R>
 struct Work {
   PrepView<R> pv;
   R* OD;            // [n][K][L]
-  R* TAU, *DTOP;    // [n][Kmax][L]
+  R* TAU, *DTOP;    // [n][Kmax][L] (FP64 form: TAU of batches with clouds or aerosols)
+  R* FIN;           // FP64 form: [n][4][L] column_tile_kernel -> column_finish_kernel
   R* PT;            // [n][Kmax][L]
   R* SC;            // [n][L]
   double* TSK;      // adjoint: [n][L]
@@ -882,14 +883,16 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
   pv.ub_k0 = (int*)carve(nn * Kmax * sizeof(int));
   pv.ub_n = (int*)carve(nn * Kmax * sizeof(int));
   pv.ub_w = (double*)carve(nn * Kmax * MAX_UBAND * sizeof(double));
-  pv.scal = (double*)carve(nn * 4 * sizeof(double));
+  pv.scal = (double*)carve(nn * PREP_SCAL * sizeof(double));
   pv.status = (int*)carve(nn * sizeof(int));
   pv.opt = s.ov.n > 0 ? (double*)carve(nn * K * OPT_NS * sizeof(double)) : nullptr;
   pv.K = K; pv.Kmax = Kmax; pv.npf = npf; pv.npa = adj ? npa : 0;
   Work<R> wk{};
   wk.pv = pv;
   wk.OD = (R*)carve(nn * K * L * sizeof(R));
-  if (mode == 3) wk.TAU = (R*)carve(nn * Kmax * L * sizeof(R));
+  constexpr bool tile = sizeof(R) == sizeof(double);   // column_tile_kernel
+  if (tile) wk.FIN = (R*)carve(nn * 4 * L * sizeof(R));
+  if (sw.rec > 0 || (adj && !tile)) wk.TAU = (R*)carve(nn * Kmax * L * sizeof(R));
   if (sw.rec > 0) {
     if (sw.kstate)
       wk.LBK = (R*)carve(nn * Kmax * (size_t)sw.rec * L * sizeof(R));
@@ -916,8 +919,7 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
     wk.TD = sw.kstate && (sw.slots || sw.cf) ? (double*)carve(nn * 2 * Kmax * sizeof(double)) : nullptr;
   }
   if (adj) {
-    wk.TAU = (R*)carve(nn * Kmax * L * sizeof(R));
-    wk.DTOP = (R*)carve(nn * Kmax * L * sizeof(R));
+    if (!tile) wk.DTOP = (R*)carve(nn * Kmax * L * sizeof(R));
     wk.PT = (R*)carve(nn * Kmax * L * sizeof(R));
     wk.SC = (R*)carve(nn * L * sizeof(R));
     wk.RA = (R*)carve(nn * nv * K * L * sizeof(R));
@@ -1056,6 +1058,43 @@ int copy_chunk(crtm_gpu_handle h, const HostCopy* hc, int p0, int n, cudaStream_
   return CRTM_GPU_SUCCESS;
 }
 
+// The column kernel (mixed form), or the tiled one and its finish (FP64 form).
+template <class R>
+int launch_column(crtm_gpu_handle h, ColumnArgs<R>& ca, cudaStream_t st) {
+  const bool ext = rts_ext_any(ca.x);
+  const dim3 gf((ca.L + 127) / 128, ca.n_chunk);
+  if constexpr (sizeof(R) == sizeof(float)) {
+    const size_t smem = column_smem_bytes<R>(ca.K, ca.Kmax);
+    if (reserve_smem(h, ext ? column_kernel<R, true> : column_kernel<R, false>, smem, "column"))
+      return CRTM_GPU_FAILURE;
+    StageScope sc(h, 2, st);
+    if (ext)
+      column_kernel<R, true><<<gf, 128, smem, st>>>(ca);
+    else
+      column_kernel<R, false><<<gf, 128, smem, st>>>(ca);
+    CK_LAUNCH(h);
+  } else {
+    const bool full = ext || ((ca.mode == 1 || ca.mode == 2) && ca.pass != 1);
+    ca.cshift = column_cshift<R>(ca.K, ca.Kmax, ca.L, ca.n_chunk, full);
+    const size_t smem = column_tile_smem_bytes<R>(ca.K, ca.Kmax, ca.cshift, full);
+    const dim3 gc((ca.L + (1 << ca.cshift) - 1) >> ca.cshift, ca.n_chunk);
+    if (reserve_smem(h, ext ? column_tile_kernel<R, true> : column_tile_kernel<R, false>, smem, "column"))
+      return CRTM_GPU_FAILURE;
+    StageScope sc(h, 2, st);
+    if (ext)
+      column_tile_kernel<R, true><<<gc, COL_THREADS, smem, st>>>(ca);
+    else
+      column_tile_kernel<R, false><<<gc, COL_THREADS, smem, st>>>(ca);
+    CK_LAUNCH(h);
+    if (ext)
+      column_finish_kernel<R, true><<<gf, 128, 0, st>>>(ca);
+    else
+      column_finish_kernel<R, false><<<gf, 128, 0, st>>>(ca);
+    CK_LAUNCH(h);
+  }
+  return CRTM_GPU_SUCCESS;
+}
+
 // mode 0 forward, 1 K-matrix, 2 adjoint
 // perm: device array of the batch profiles the pipeline runs, in order
 // (b->n_profiles of them), or null for all of the batch's profiles in its
@@ -1158,7 +1197,6 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
   bv.perm = perm;
   constexpr int NPF = Tune<G, R>::FWD, NPA = Tune<G, R>::AD;
   const size_t prep_smem = prep_smem_bytes<G>(K, Kmax);
-  const size_t col_smem = column_smem_bytes<R>(K, Kmax);
   // channels per map CTA: 16 (more resident CTAs hide the tile loads; C2:
   // 6.4 ms against 7.4 ms with 32 and 8.1 ms with 8), fewer if the tiles exceed
   // the shared-memory budget (CRTM_GPU_MAP_CHANNELS: 8, 16 or 32 overrides;
@@ -1168,8 +1206,6 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
   const size_t map_smem = map_smem_bytes<R>(K, Kmax, nv, map_ct);
   constexpr size_t fwd_smem = fwd_smem_bytes<G, R, NPF>();
   if (reserve_smem(h, absorb_fwd_kernel<G, R, NPF>, fwd_smem, "absorb_fwd") ||
-      reserve_smem(h, column_kernel<R, false>, col_smem, "column") ||
-      reserve_smem(h, column_kernel<R, true>, col_smem, "column") ||
       reserve_smem(h, map_kernel<R>, map_smem, "map"))
     return CRTM_GPU_FAILURE;
   const bool ho_only = [&] {
@@ -1201,7 +1237,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
     ColumnArgs<R> ca{};
     ca.K = K; ca.L = L; ca.Kmax = Kmax; ca.p_begin = p0; ca.n_chunk = n; ca.mode = mode;
     ca.b = bv; ca.sp = s.spec; ca.pv = w.pv; ca.OD = w.OD;
-    ca.TAU = w.TAU; ca.DTOP = w.DTOP; ca.PT = w.PT; ca.SC = w.SC;
+    ca.TAU = w.TAU; ca.DTOP = w.DTOP; ca.FIN = w.FIN; ca.PT = w.PT; ca.SC = w.SC;
     ca.seed = seed; ca.radiance = rts->radiance; ca.bt = rts->brightness_temperature;
     ca.tsk = mode == 1 ? kk->water_temperature : (mode == 2 ? w.TSK : nullptr);
     ca.ek = mode == 1 ? kk->surface_emissivity : nullptr;
@@ -1222,15 +1258,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
       ca.n_aerosols = b->max_aerosols > 0 ? b->n_aerosols : nullptr;
       ca.TODc = w.TODc; ca.CB = w.CB; ca.cover = w.cover;
     }
-    dim3 gc((L + 127) / 128, n);
-    {
-      StageScope sc(h, 2, st);
-      if (rts_ext_any(ca.x))
-        column_kernel<R, true><<<gc, 128, col_smem, st>>>(ca);
-      else
-        column_kernel<R, false><<<gc, 128, col_smem, st>>>(ca);
-      CK_LAUNCH(h);
-    }
+    if (int rc = launch_column<R>(h, ca, st)) return rc;
     if (scat) {   // layer optics, then the adding from the surface (and its adjoint)
       ScatterArgs<R> sa{};
       sa.K = K; sa.L = L; sa.Kmax = Kmax; sa.p_begin = p0; sa.n_chunk = n;
@@ -1309,12 +1337,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
         }
         {
           ca.pass = 2;
-          StageScope sc(h, 2, st);
-          if (rts_ext_any(ca.x))
-        column_kernel<R, true><<<gc, 128, col_smem, st>>>(ca);
-      else
-        column_kernel<R, false><<<gc, 128, col_smem, st>>>(ca);
-          CK_LAUNCH(h);
+          if (int rc = launch_column<R>(h, ca, st)) return rc;
         }
         if (sw.slots || sw.cf) {   // species and cloud-fraction Jacobians: cover chain rule, seed, outputs
           StageScope sc(h, 9, st);

@@ -7,13 +7,13 @@
 //                      partial-derivative table D; mapping bands for the adjoint
 //   absorb_fwd_kernel  one thread per (channel, NPF profiles): reference-layer
 //                      OD = sum C*X (ODPS_AtmAbsorption.f90:169-208)
-//   column_kernel      one CTA per (profile, 32 channels), one warp per channel,
-//                      layers across lanes: clamp + path + level interpolation
-//                      (ODPS_AtmAbsorption.f90:213-254), Planck, Emission
-//                      (Emission_Module.f90:54-174) as affine warp scans, Planck
-//                      inversion; for K/AD the Emission adjoint
-//                      (Emission_Module.f90:280-395) and the optical-depth path
-//                      adjoint (ODPS_AtmAbsorption.f90:487-540), also as scans
+//   column_kernel      one thread per (profile, channel): clamp + path + level
+//                      interpolation (ODPS_AtmAbsorption.f90:213-254), Planck,
+//                      Emission (Emission_Module.f90:54-174), Planck inversion;
+//                      for K/AD the Emission adjoint (Emission_Module.f90:280-395)
+//                      and the optical-depth path adjoint
+//                      (ODPS_AtmAbsorption.f90:487-540); FP64 form:
+//                      column_tile_kernel, column_finish_kernel
 //   absorb_ad_kernel   one thread per (channel, NPA profiles): coefficient x
 //                      predictor-partial contraction and reverse running sums
 //                      (ODPS_AtmAbsorption.f90:543-598, ODPS_Predictor.f90:1783-2643)
@@ -258,6 +258,8 @@ struct RefSums {
   const double* gatzp_ref;  // [Jm][K]
 };
 
+constexpr int PREP_SCAL = 8;   // per-profile scalars (PrepView::scal)
+
 template <class R>
 struct PrepView {
   R* Xg;               // [ceil(n/npf)][K][NS][npf]
@@ -273,7 +275,8 @@ struct PrepView {
   int* ub_k0;          // [n][Kmax] first reference layer mapping to user layer ku
   int* ub_n;           // [n][Kmax]
   double* ub_w;        // [n][Kmax][MAX_UBAND]
-  double* scal;        // [n][4]: sec_surface, u = cos(sensor zenith)
+  double* scal;        // [n][PREP_SCAL]: sec_surface, u = cos(sensor zenith), their reciprocals, the
+                       // surface temperature (coverage-weighted)
   int* status;         // [n]
   double* opt;         // [n][K][OPT_NS] OPTRAN predictor state, or null (no OPTRAN channels)
   int K, Kmax, npf, npa;
@@ -497,8 +500,13 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_kernel(SensorTables S, RefS
       atomicMin(&sLo[c], i); atomicMax(&sHi[c], i);
     }
     if (tid == 0) {
-      pv.scal[(size_t)p * 4 + 0] = geo.sec_surface;
-      pv.scal[(size_t)p * 4 + 1] = geo.cos_sensor;
+      double* sc = pv.scal + (size_t)p * PREP_SCAL;
+      sc[0] = geo.sec_surface;
+      sc[1] = geo.cos_sensor;
+      sc[2] = 1.0 / geo.sec_surface;
+      sc[3] = 1.0 / geo.cos_sensor;
+      sc[4] = b.land_cov[gp] * b.land_t[gp] + b.water_cov[gp] * b.water_t[gp] +
+              b.snow_cov[gp] * b.snow_t[gp] + b.ice_cov[gp] * b.ice_t[gp];
     }
   }
   // ---- user layer ku <- reference layers mapping to it (Map_Input adjoint)
@@ -718,7 +726,8 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) absorb_fwd_kernel(int K, int k
 }
 
 // ---------------------------------------------------------------------------
-// 3. column: one thread per (profile, channel), two passes over the user layers.
+// 3. column, mixed form: one thread per (profile, channel), two passes over the
+//    user layers (the FP64 form: 3b).
 //    mode 0 forward, 1 K-matrix, 2 adjoint, 3 layer optical depths only.
 //
 //    Pass 1 (top down) follows the forward model: OD path and its interpolation
@@ -737,9 +746,12 @@ struct ColumnArgs {
   SpecView sp;
   PrepView<R> pv;
   R* OD;                  // [n][K][L]: in reference ODs, out (K/AD) unit-seed OD adjoint
-  R* TAU, *DTOP;          // [n][Kmax][L] scratch: layer OD and downwelling at the layer top
+  R* TAU, *DTOP;          // [n][Kmax][L] scratch: layer OD and (mixed form) downwelling at the layer top
   R* PT;                  // [n][Kmax][L] unit-seed Planck part of the temperature adjoint
   R* SC;                  // [n][L] adjoint seed dBT/dR * seed
+  int cshift;             // FP64 form: channels per CTA, 1 << cshift
+  R* FIN;                 // FP64 form: [n][4][L] for the finish: TOA radiance, column transmittance,
+                          // downwelling at the surface, atmospheric upwelling
   const double* seed;     // [P][L] or null (=1)
   double* radiance, *bt;  // [P][L]
   double* tsk, *ek;       // K-matrix: [P][L] water temperature, emissivity; adjoint: tsk is [n][L]
@@ -843,15 +855,14 @@ __global__ void __launch_bounds__(128) column_kernel(ColumnArgs<R> a) {
   __syncthreads();
   if (l >= L) return;
   const size_t pl = (size_t)gp * L + l;
-  const double* sc = a.pv.scal + (size_t)p * 4;
-  const R inv_sec = R(1.0 / sc[0]);
-  const R inv_u = R(1.0 / sc[1]);
+  const double* sc = a.pv.scal + (size_t)p * PREP_SCAL;
+  const R inv_sec = R(sc[2]);
+  const R inv_u = R(sc[3]);
   const double c1d = a.sp.c1[l], c2d = a.sp.c2[l], b1d = a.sp.b1[l], b2d = a.sp.b2[l];
   const R c1 = R(c1d), c2 = R(c2d), b1 = R(b1d), b2 = R(b2d);
   const double e = a.b.emissivity[pl];
   const R re = R(e), rr = R(1.0 - e);
-  const double tsd = a.b.land_cov[gp] * a.b.land_t[gp] + a.b.water_cov[gp] * a.b.water_t[gp] +
-                     a.b.snow_cov[gp] * a.b.snow_t[gp] + a.b.ice_cov[gp] * a.b.ice_t[gp];
+  const double tsd = sc[4];
   // surface Planck radiance and its temperature derivative in R (the Planck
   // inversion at the end stays in FP64)
   const R ted = b1 + b2 * R(tsd);
@@ -1055,6 +1066,488 @@ __global__ void __launch_bounds__(128) column_kernel(ColumnArgs<R> a) {
     zero_row(x.lod, pl, Kmax, Ku);
     zero_row(x.upw, pl, Kmax, Ku);
     zero_row(x.ovc, pl, Kmax, Ku);
+  }
+  const double seed = a.seed ? a.seed[pl] : 1.0;
+  const double scale = dtdr * seed;
+  a.SC[(size_t)p * L + l] = R(scale);
+  const R dden = ted * (eed - R(1));
+  const R dBs = c1 * c2 * eed * b2 / (dden * dden);
+  // surface temperature: Ts = sum of the coverage-weighted cover temperatures
+  // (CRTM_Compute_SurfaceT), so each cover's adjoint is its coverage x dBT/dTs
+  const double ts_ad = double(dBs) * Bs_b * scale;
+  // emissivity model (water coverage 1): de/dT adds to the water temperature
+  // adjoint, de/dv gives the wind speed's (CRTM_Compute_IRSSEM_AD)
+  const double e_ad = scale * e_b;   // emissivity_AD - reflectivity_AD
+  const double ts_e = a.sfc_et ? e_ad * a.sfc_et[pl] : 0.0;
+  if (a.mode == 1) {
+    a.tsk[pl] = a.b.water_cov[gp] * ts_ad + ts_e;
+    if (a.tsk_land) a.tsk_land[pl] = a.b.land_cov[gp] * ts_ad;
+    if (a.tsk_snow) a.tsk_snow[pl] = a.b.snow_cov[gp] * ts_ad;
+    if (a.tsk_ice) a.tsk_ice[pl] = a.b.ice_cov[gp] * ts_ad;
+    a.ek[pl] = e_ad;
+    if (a.wind_k) a.wind_k[pl] = e_ad * a.sfc_ev[pl];
+  } else {
+    a.tsk[(size_t)p * L + l] = ts_ad + ts_e;
+    if (a.wind_k) a.wind_k[(size_t)p * L + l] = e_ad * a.sfc_ev[pl];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// 3b. column, FP64 form: one CTA per (profile, tile of channels), the same
+//    arithmetic.  Only a few additions and multiplications are sequential over
+//    the layers: one thread per channel runs those recursions on values in
+//    shared memory, and all of the CTA's threads evaluate what is independent
+//    per layer (interpolation, exponentials, Planck radiances and derivatives,
+//    the layer adjoints, the reference levels' path adjoints).
+//
+//    Bound: FP64 issue (an exponential is some 25 instructions of 64 clocks
+//    each per scheduler), so two exponentials a layer, reciprocals instead of
+//    divisions, and the transmittance above a layer from the recursion.  A
+//    thread per (profile, channel) kept one of an SM's four schedulers busy for
+//    a single 22-channel profile (246 us, now 58) and evaluated the exponentials
+//    once per pass (K-matrix columns of 250 x 616: 5.6 ms, now 4.3).  In the
+//    mixed form the recursions' latency weighs more than the exponentials: the
+//    tile took 7.3 ms for 1000 x 2211 K-matrix columns against 3.4 ms, so it
+//    keeps the thread per pair.
+// ---------------------------------------------------------------------------
+constexpr int COL_THREADS = 256;
+
+// Rows (of cw + 1 values; the odd stride keeps both the rows and the columns
+// free of bank conflicts) of a column CTA's shared memory: path, and per
+// layer transmittance, Planck radiance, optical depth; with adjoints or
+// layer components the upwelling radiance, the transmittance below and the
+// Planck derivative.
+CRTM_HD int column_rows(int K, int Kmax, bool full) {
+  return (K > Kmax ? K : Kmax) + 1 + Kmax * (full ? 6 : 3);
+}
+template <class R>
+inline size_t column_tile_smem_bytes(int K, int Kmax, int cshift, bool full) {
+  const int cw = 1 << cshift;
+  return sizeof(R) * ((size_t)column_rows(K, Kmax, full) * (cw + 1) + 2 * (size_t)Kmax + 1 + 8 * cw) +
+         sizeof(int) * (2 * (size_t)(Kmax + 1) + 2 * (size_t)(K + 1) + (size_t)((K + 31) / 32) * cw) + 16;
+}
+
+// Channels per column CTA (log2).  32 fill the recursions' warp; fewer where
+// the tile would leave less than two CTAs per SM (so that one CTA's
+// recursions overlap another's exponentials), and down to 4 while the launch
+// has fewer CTAs than 2 per SM: a CTA's time is nearly proportional to its
+// tile in the FP64 form (one 22-channel profile).
+template <class R>
+inline int column_cshift(int K, int Kmax, int L, int n, bool full) {
+  int c = 5;
+  while (c > 2 && column_tile_smem_bytes<R>(K, Kmax, c, full) > 112 * 1024) c--;
+  while (c > 2 && (long long)n * ((L + (1 << c) - 1) >> c) < 152 * 2) c--;
+  return c;
+}
+
+// EXT: the call asks for further RTSolution components (a.x); without them
+// the component code compiles out.
+template <class R, bool EXT>
+__global__ void __launch_bounds__(COL_THREADS) column_tile_kernel(ColumnArgs<R> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int K = a.K, L = a.L, Kmax = a.Kmax;
+  const int p = blockIdx.y, gp = batch_profile(a.b, a.p_begin + p);
+  const int tid = threadIdx.x, cw = 1 << a.cshift, CS = cw + 1;
+  const int c = tid & (cw - 1), r0 = tid >> a.cshift, rstep = COL_THREADS >> a.cshift;
+  const int l0 = blockIdx.x << a.cshift, l = l0 + c;
+  const int st = a.pv.status[p];
+  const int Ku = a.b.n_layers[gp];
+  const RtsExt x = EXT ? a.x : RtsExt{};
+  if (st != 0) {   // column_finish_kernel writes the profile's zeros
+    if (tid < cw && l < L) {
+      const size_t pl = (size_t)gp * L + l;
+      zero_row(x.lod, pl, Kmax, 0);
+      zero_row(x.upw, pl, Kmax, 0);
+      zero_row(x.ovc, pl, Kmax, 0);
+    }
+    return;
+  }
+  const bool adj = (a.mode == 1 || a.mode == 2) && a.pass != 1;   // this launch computes adjoints
+  const bool full = adj || EXT;
+  // a profile with clouds or aerosols (solved by the scattering kernels):
+  // every profile of a forward launch in mode 3, those with clouds or
+  // aerosols in the K-matrix / adjoint launches around the scattering kernels
+  const bool scat_p = a.mode == 3 ||
+                      ((a.pass == 1 || a.pass == 2) &&
+                       ((a.n_clouds && a.n_clouds[gp] > 0) || (a.n_aerosols && a.n_aerosols[gp] > 0)));
+  const int KP = K > Kmax ? K : Kmax;
+  R* sP = reinterpret_cast<R*>(smem_raw);       // [KP+1][CS] OD path at the reference levels, then the
+                                                // downwelling at the layer tops, then the levels' path adjoints
+  R* sT = sP + (size_t)(KP + 1) * CS;           // [Kmax][CS] layer transmittance
+  R* sB = sT + (size_t)Kmax * CS;               // [Kmax][CS] Planck radiance
+  R* sTau = sB + (size_t)Kmax * CS;             // [Kmax][CS] optical depth; transmittance above; dR/dtau
+  R* sU = sTau + (size_t)Kmax * CS;             // [Kmax][CS] upwelling at the layer bottom (full)
+  R* sQ = sU + (full ? (size_t)Kmax * CS : 0);  // [Kmax][CS] transmittance below the layer (full)
+  R* sD = sQ + (full ? (size_t)Kmax * CS : 0);  // [Kmax][CS] dB/dT (full)
+  R* spec = reinterpret_cast<R*>(smem_raw) + (size_t)column_rows(K, Kmax, full) * CS;   // [8][cw]
+  R* facd = spec + 8 * cw;                      // [Kmax+1] interpolation factors
+  R* tus = facd + Kmax + 1;                     // [Kmax] layer temperatures
+  int* k1s = reinterpret_cast<int*>(tus + Kmax);         // [Kmax+1]
+  int* k2s = k1s + (Kmax + 1);
+  int* ilos = k2s + (Kmax + 1);                          // [K+1]
+  int* ihis = ilos + (K + 1);
+  unsigned* flags = reinterpret_cast<unsigned*>(ihis + (K + 1));   // [ceil(K/32)][cw] clamped layers
+  const bool chan = l < L;
+  const size_t pl = (size_t)gp * L + (chan ? l : 0);
+  R* od = a.OD + (size_t)p * K * L + l;
+  // ---- stage the tables and the reference optical depths
+  {
+    const double* tug = a.b.temperature + (size_t)gp * Kmax;
+    for (int i = tid; i < Kmax; i += COL_THREADS) tus[i] = R(i < Ku ? tug[i] : 0.0);
+    const int* k1g = a.pv.ulev_k1 + (size_t)p * (Kmax + 1);
+    const int* k2g = a.pv.ulev_k2 + (size_t)p * (Kmax + 1);
+    const double* fg = a.pv.ulev_fac + (size_t)p * (Kmax + 1);
+    for (int i = tid; i <= Ku; i += COL_THREADS) { k1s[i] = k1g[i]; k2s[i] = k2g[i]; facd[i] = R(fg[i]); }
+    if (adj) {
+      const int* ilg = a.pv.rlev_ilo + (size_t)p * (K + 1);
+      const int* ihg = a.pv.rlev_ihi + (size_t)p * (K + 1);
+      for (int i = tid; i <= K; i += COL_THREADS) { ilos[i] = ilg[i]; ihis[i] = ihg[i]; }
+    }
+    for (int k = r0; k < K; k += rstep) sP[(k + 1) * CS + c] = chan ? od[(size_t)k * L] : R(0);
+    if (tid < cw && chan) {
+      sP[c] = R(0);
+      spec[c] = R(a.sp.c1[l]); spec[cw + c] = R(a.sp.c2[l]);
+      spec[2 * cw + c] = R(a.sp.b1[l]); spec[3 * cw + c] = R(a.sp.b2[l]);
+    }
+  }
+  const double* sc = a.pv.scal + (size_t)p * PREP_SCAL;
+  const R inv_sec = R(sc[2]);
+  const R inv_u = R(sc[3]);
+  __syncthreads();
+  // one value per channel and layer of a serial pass is fetched NB layers ahead
+  constexpr int NB = 8;
+  // ---- OD path at the reference levels (top down)
+  if (tid < cw) {
+    R path = R(0);
+    unsigned word = 0u;
+    for (int k0 = 0; k0 < K; k0 += NB) {
+      R v[NB];
+#pragma unroll
+      for (int j = 0; j < NB; j++) v[j] = sP[min(k0 + j + 1, K) * CS + c];
+#pragma unroll
+      for (int j = 0; j < NB; j++)
+        if (k0 + j < K) {
+          if (v[j] < R(0) || v[j] > R(MAX_OD)) word |= 1u << ((k0 + j) & 31);
+          path += clamp_od(v[j]);
+          v[j] = path;
+        }
+#pragma unroll
+      for (int j = 0; j < NB; j++)
+        if (k0 + j < K) sP[(k0 + j + 1) * CS + c] = v[j];
+      if (((k0 + NB) & 31) == 0 || k0 + NB >= K) {
+        flags[(k0 >> 5) * cw + c] = word;
+        word = 0u;
+      }
+    }
+  }
+  __syncthreads();
+  // ---- user levels and layers: optical depth, transmittance, Planck radiance
+  {
+    const R c1 = spec[c], c2 = spec[cw + c], b1 = spec[2 * cw + c], b2 = spec[3 * cw + c];
+    auto level = [&](int i) {   // OD path at user level i
+      const int k = k2s[i];
+      const R path_cur = sP[k * CS + c];
+      if (k1s[i] == k) return path_cur;
+      const R path_prev = sP[(k - 1) * CS + c];
+      return path_prev + (path_cur - path_prev) * facd[i];
+    };
+    const size_t cs = (size_t)p * Kmax * L + l;
+    for (int ku = r0; ku < Ku; ku += rstep) {
+      const R tau = (level(ku + 1) - level(ku)) * inv_sec;
+      sTau[ku * CS + c] = tau;
+      if ((a.mode == 3 || a.pass == 1) && chan) a.TAU[cs + (size_t)ku * L] = tau;
+      if (a.mode == 3 || (a.pass == 1 && scat_p)) continue;
+      // (reciprocals: an FP64 division costs as much as ten multiplications)
+      const R rte = R(1) / (b1 + b2 * tus[ku]);
+      const R ee = exp(c2 * rte);
+      const R rem1 = R(1) / (ee - R(1));
+      sT[ku * CS + c] = exp(-tau * inv_u);
+      sB[ku * CS + c] = c1 * rem1;
+      if (adj) {
+        const R rden = rte * rem1;
+        sD[ku * CS + c] = c1 * c2 * b2 * ee * rden * rden;
+      }
+    }
+  }
+  __syncthreads();
+  // rows of the CTA's channels out of shared memory (v[ku][c]) to o[pl][Kmax], layers across lanes
+  auto rows_out = [&](double* o, const R* v) {
+    for (int cc = tid >> 5; cc < cw && l0 + cc < L; cc += COL_THREADS / 32) {
+      double* r = o + ((size_t)gp * L + l0 + cc) * Kmax;
+      for (int ku = tid & 31; ku < Kmax; ku += 32) r[ku] = ku < Ku && v ? double(v[ku * CS + cc]) : 0.0;
+    }
+  };
+  if (x.lod && a.pass != 2) {
+    rows_out(x.lod, sTau);
+    __syncthreads();   // the recursions below reuse the rows
+  }
+  if (a.mode == 3 || (a.pass == 1 && scat_p)) {
+    // Emission-only components zero; the scattering kernels fill the rest
+    if (x.upw) rows_out(x.upw, nullptr);
+    if (x.ovc) rows_out(x.ovc, nullptr);
+    return;
+  }
+  // ---- downwelling, column transmittance, atmospheric upwelling (top down)
+  const double e = chan ? a.b.emissivity[pl] : 1.0;
+  const R re = R(e), rr = R(1.0 - e);
+  R Dn = R(0), Tn = R(1), src = R(0), Bs = R(0);
+  const bool want_ovc = x.ovc && a.pass != 2 && !scat_p;
+  if (tid < cw && chan) {
+    const R c1 = spec[c], c2 = spec[cw + c], b1 = spec[2 * cw + c], b2 = spec[3 * cw + c];
+    // surface Planck radiance in R (the Planck inversion stays in FP64)
+    const R ted = b1 + b2 * R(sc[4]);
+    const R eed = exp(c2 / ted);
+    Bs = c1 / (eed - R(1));
+    R rad_down = R(a.sp.cbr[l]), tr = R(1);
+    for (int k0 = 0; k0 < Ku; k0 += NB) {
+      R tv[NB], Bv[NB];
+#pragma unroll
+      for (int j = 0; j < NB; j++) {
+        const int k = min(k0 + j, Ku - 1);
+        tv[j] = sT[k * CS + c]; Bv[j] = sB[k * CS + c];
+      }
+#pragma unroll
+      for (int j = 0; j < NB; j++)
+        if (k0 + j < Ku) {
+          const R t = tv[j], B = Bv[j];
+          if (want_ovc) sU[(k0 + j) * CS + c] = src + tr * B;   // a black cloud filling the layer
+          const R Bt = B * (R(1) - t);
+          if (adj) {
+            sP[(k0 + j) * CS + c] = rad_down;
+            sTau[(k0 + j) * CS + c] = tr;   // TOA to the top of this layer
+          }
+          if (EXT || a.mode == 0) src += tr * Bt;
+          tr *= t;
+          rad_down = rad_down * t + Bt;
+        }
+    }
+    Dn = rad_down;
+    Tn = tr;
+  }
+  if (want_ovc) {
+    __syncthreads();
+    rows_out(x.ovc, sU);
+    __syncthreads();
+  }
+  if (a.pass == 1) return;   // a clear profile around the scattering kernels: pass 2 finishes it
+  const bool want_upw = x.upw && !scat_p;
+  R* fin = a.FIN + (size_t)p * 4 * L + l;
+  if (a.mode == 0) {
+    if (tid < cw && chan) {
+      fin[0] = src + Tn * (re * Bs + rr * Dn);
+      fin[(size_t)L] = Tn;
+      fin[2 * (size_t)L] = Dn;
+      fin[3 * (size_t)L] = src;
+      if (want_upw) {   // upwelling at each layer's bottom, surface to top
+        R U = re * Bs + rr * Dn;
+        for (int ku = Ku - 1; ku >= 0; ku--) {
+          const R t = sT[ku * CS + c], B = sB[ku * CS + c];
+          sU[ku * CS + c] = U;
+          U = t * U + B * (R(1) - t);
+        }
+      }
+    }
+    if (want_upw) {
+      __syncthreads();
+      rows_out(x.upw, sU);
+    }
+    return;
+  }
+  // ---- upwelling and transmittance below each layer (bottom up)
+  if (tid < cw && chan) {
+    R U = re * Bs + rr * Dn;
+    R P = R(1);                 // transmittance of the layers below the current one
+    for (int k0 = Ku - 1; k0 >= 0; k0 -= NB) {
+      R tv[NB], Bv[NB];
+#pragma unroll
+      for (int j = 0; j < NB; j++) {
+        const int k = max(k0 - j, 0);
+        tv[j] = sT[k * CS + c]; Bv[j] = sB[k * CS + c];
+      }
+#pragma unroll
+      for (int j = 0; j < NB; j++)
+        if (k0 - j >= 0) {
+          const int at = (k0 - j) * CS + c;
+          const R t = tv[j], B = Bv[j];
+          sU[at] = U;
+          sQ[at] = P;
+          U = B + t * (U - B);
+          P *= t;
+        }
+    }
+    fin[0] = U;
+    fin[(size_t)L] = Tn;
+    fin[2 * (size_t)L] = Dn;
+    fin[3 * (size_t)L] = src;
+    spec[4 * cw + c] = rr * Tn;   // downwelling adjoint at the surface (unit seed)
+  }
+  __syncthreads();
+  if (want_upw) rows_out(x.upw, sU);
+  // ---- Emission adjoint of each layer (unit seed)
+  {
+    const R down0 = spec[4 * cw + c];
+    double wcloud = 0.0;   // weight of the cloudy column
+    const bool scat = scat_p;
+    if (scat) wcloud = a.cover[p] < 0.0 ? 1.0 : a.cover[p];
+    const R wclr = R(1.0 - wcloud), wcl = R(wcloud);
+    const size_t cs = (size_t)p * Kmax * L + l;
+    if (chan)
+      for (int ku = r0; ku < Kmax; ku += rstep) {
+        if (ku >= Ku) {
+          a.PT[cs + (size_t)ku * L] = R(0);
+          continue;
+        }
+        const int at = ku * CS + c;
+        const R t = sT[at], B = sB[at], U = sU[at], P = sQ[at], Dtop = sP[at], dB = sD[at];
+        // the upwelling (Emission_AD first loop) and the downwelling part (second loop)
+        const R up = sTau[at], dad = down0 * P;
+        R tod = -(up * (U - B) + dad * (Dtop - B)) * (t * inv_u);
+        R ptv = dB * ((up + dad) * (R(1) - t));
+        if (scat) {
+          ptv = wclr * ptv + wcl * a.PT[cs + (size_t)ku * L];
+          tod = wclr * tod + wcl * a.TODc[cs + (size_t)ku * L];
+        }
+        a.PT[cs + (size_t)ku * L] = ptv;
+        sTau[at] = tod;
+      }
+  }
+  __syncthreads();
+  // ---- path adjoint of each reference level: the user levels whose bracket
+  // touches it, bottom up (ODPS_AtmAbsorption.f90:519-530 and
+  // Interpolate_Profile_F1_AD)
+  for (int j = 1 + r0; j <= K; j += rstep) {
+    R pa = R(0);
+    for (int i = ihis[j]; i >= ilos[j]; i--) {
+      R v = R(0);   // user level i's path adjoint
+      if (i < Ku) v = -sTau[i * CS + c] * inv_sec;
+      if (i > 0) v += sTau[(i - 1) * CS + c] * inv_sec;
+      const int ka = k1s[i], kb = k2s[i];
+      const R f = facd[i];
+      if (ka == kb) pa += v;
+      else if (ka == j) pa += (R(1) - f) * v;
+      else if (kb == j) pa += f * v;
+    }
+    sP[j * CS + c] = pa;
+  }
+  __syncthreads();
+  // ---- OD adjoints: the sum of the path adjoints below, zero where clamped
+  if (tid < cw && chan) {
+    R suffix = R(0);
+    for (int k0 = K - 1; k0 >= 0; k0 -= NB) {
+      R v[NB];
+#pragma unroll
+      for (int j = 0; j < NB; j++) v[j] = sP[(max(k0 - j, 0) + 1) * CS + c];
+#pragma unroll
+      for (int j = 0; j < NB; j++)
+        if (k0 - j >= 0) {
+          const int k = k0 - j;
+          suffix += v[j];
+          od[(size_t)k * L] = (flags[(k >> 5) * cw + c] >> (k & 31)) & 1u ? R(0) : suffix;
+        }
+    }
+  }
+}
+
+// The rest of the FP64 form's column, one thread per (profile, channel): the Planck
+// inversion, surface derivatives and RTSolution components, in FP64.  Its own
+// kernel because the inversion is some hundred FP64 instructions per channel,
+// which one warp of a column CTA would issue at a quarter of the SM's rate.
+template <class R, bool EXT>
+__global__ void __launch_bounds__(128) column_finish_kernel(ColumnArgs<R> a) {
+  const int L = a.L;
+  const int p = blockIdx.y, gp = batch_profile(a.b, a.p_begin + p);
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  const int st = a.pv.status[p];
+  if (l == 0 && a.status) a.status[gp] = st;
+  if (l >= L) return;
+  const size_t pl = (size_t)gp * L + l;
+  const RtsExt x = EXT ? a.x : RtsExt{};
+  auto ext_scalars = [&](double e, double up, double down, double bs) {
+    if (x.emis) x.emis[pl] = e;
+    if (x.up) x.up[pl] = up;
+    if (x.down) x.down[pl] = down;
+    if (x.bs) x.bs[pl] = bs;
+  };
+  if (st != 0) {
+    a.radiance[pl] = 0.0;
+    a.bt[pl] = 0.0;
+    ext_scalars(0.0, 0.0, 0.0, 0.0);
+    if (x.tb_clear) x.tb_clear[pl] = 0.0;
+    if (x.r_clear) x.r_clear[pl] = 0.0;
+    if (x.tcc) x.tcc[pl] = 0.0;
+    if (x.sod) x.sod[pl] = 0.0;
+    if (x.nfs) x.nfs[pl] = 0;
+    if (a.mode == 1) { a.tsk[pl] = 0.0; a.ek[pl] = 0.0; }
+    if (a.mode == 1 || a.mode == 2) a.SC[(size_t)p * L + l] = R(0);
+    if (a.mode == 2) a.tsk[(size_t)p * L + l] = 0.0;
+    if (a.wind_k) a.wind_k[a.mode == 1 ? pl : (size_t)p * L + l] = 0.0;
+    return;
+  }
+  const bool scat = a.mode == 3 ||
+                    ((a.pass == 1 || a.pass == 2) &&
+                     ((a.n_clouds && a.n_clouds[gp] > 0) || (a.n_aerosols && a.n_aerosols[gp] > 0)));
+  const double e = a.b.emissivity[pl];
+  if (a.mode == 3 || a.pass == 1) {
+    if (scat) {
+      ext_scalars(e, 0.0, 0.0, 0.0);
+      if (x.sod) x.sod[pl] = 0.0;
+    }
+    return;
+  }
+  const double c1d = a.sp.c1[l], c2d = a.sp.c2[l], b1d = a.sp.b1[l], b2d = a.sp.b2[l];
+  const R c1 = R(c1d), c2 = R(c2d), b1 = R(b1d), b2 = R(b2d);
+  const R ted = b1 + b2 * R(a.pv.scal[(size_t)p * PREP_SCAL + 4]);
+  const R eed = exp(c2 / ted);
+  const R Bs = c1 / (eed - R(1));
+  const R* fin = a.FIN + (size_t)p * 4 * L + l;
+  const R U = fin[0], Tn = fin[(size_t)L], Dn = fin[2 * (size_t)L], src = fin[3 * (size_t)L];
+  const int nsu = a.n_streams ? a.n_streams[gp] : 0;
+  if (a.mode == 0) {
+    const double Rd = double(U);
+    const double btv = planck_temperature(c1d, c2d, b1d, b2d, Rd);
+    a.radiance[pl] = Rd;
+    a.bt[pl] = btv;
+    ext_scalars(e, double(src), double(Dn), double(Bs));
+    if (x.tb_clear) x.tb_clear[pl] = btv;   // no clouds (CRTM_Forward_Module.f90:1115-1119)
+    if (x.r_clear) x.r_clear[pl] = Rd;
+    if (x.tcc) x.tcc[pl] = 0.0;
+    if (x.sod) x.sod[pl] = 0.0;
+    if (x.nfs) x.nfs[pl] = nsu > 0 ? nsu + 2 : 0;
+    return;
+  }
+  double wcloud = 0.0;   // weight of the cloudy column
+  if (scat) wcloud = a.cover[p] < 0.0 ? 1.0 : a.cover[p];
+  // ---- TOA radiance, brightness temperature and the adjoint seed; the
+  // surface derivatives for a unit radiance seed (emissivity with the
+  // reflectivity 1 - e, and the surface Planck radiance)
+  double Rd = double(U);
+  double e_b = double(Tn) * (double(Bs) - double(Dn));
+  double Bs_b = e * double(Tn);
+  if (scat) {
+    const double* cb = a.CB + (size_t)p * 4 * L + l;
+    Rd = (1.0 - wcloud) * Rd + wcloud * cb[0];
+    e_b = (1.0 - wcloud) * e_b + wcloud * cb[(size_t)L];
+    Bs_b = (1.0 - wcloud) * Bs_b + wcloud * cb[2 * (size_t)L];
+  }
+  a.radiance[pl] = Rd;
+  double btv, dtdr;
+  planck_temperature_with_dR(c1d, c2d, b1d, b2d, Rd, &btv, &dtdr);
+  a.bt[pl] = btv;
+  // further RTSolution components: the K-matrix and adjoint fill R_clear and
+  // Tb_clear for fractional profiles only (CRTM_K_Matrix_Module.f90:1328-1336)
+  if (scat) {
+    const bool frac = a.cover[p] >= 0.0;
+    const double Rc = double(U);
+    if (x.tcc) x.tcc[pl] = frac ? a.cover[p] : 0.0;
+    if (x.r_clear) x.r_clear[pl] = frac ? Rc : 0.0;
+    if (x.tb_clear) x.tb_clear[pl] = frac ? planck_temperature(c1d, c2d, b1d, b2d, Rc) : 0.0;
+  } else {
+    ext_scalars(e, double(src), double(Dn), double(Bs));
+    if (x.tcc) x.tcc[pl] = 0.0;
+    if (x.r_clear) x.r_clear[pl] = 0.0;
+    if (x.tb_clear) x.tb_clear[pl] = 0.0;
+    if (x.sod) x.sod[pl] = 0.0;
+    if (x.nfs) x.nfs[pl] = nsu > 0 ? nsu + 2 : 0;
   }
   const double seed = a.seed ? a.seed[pl] : 1.0;
   const double scale = dtdr * seed;

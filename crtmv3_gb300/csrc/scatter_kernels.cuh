@@ -192,7 +192,7 @@ __device__ __forceinline__ CloudyColumn column_inputs(const ScatterArgs<R>& a, i
   c.nleg = ns > 0 ? ns : stream_rule_nleg(a.maxreff[p], a.sp.wn[l]);
   c.microwave = a.microwave != 0;
   c.freq = a.microwave ? a.sp.freq[l] : a.sp.wn[l];
-  c.mu_sensor = a.pv.scal[(size_t)p * 4 + 1];
+  c.mu_sensor = a.pv.scal[(size_t)p * PREP_SCAL + 1];
   const size_t pl = (size_t)gp * a.L + l;
   c.emissivity = a.b.emissivity[pl];
   c.c1 = a.sp.c1[l]; c.c2 = a.sp.c2[l]; c.b1 = a.sp.b1[l]; c.b2 = a.sp.b2[l];
