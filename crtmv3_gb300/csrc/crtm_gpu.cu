@@ -1427,8 +1427,11 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
     } else {
       StageScope sc(h, 5, st);
       const long long rows_ra = (long long)n * nv * K;
-      channel_sum_kernel<R><<<(unsigned)((rows_ra * 32 + 255) / 256), 256, 0, st>>>(
-          w.RA, nullptr, 1, rows_ra, L, w.ras);
+      if constexpr (sizeof(R) == sizeof(float))
+        channel_sum_fixed_kernel<<<(unsigned)((rows_ra * 32 + 255) / 256), 256, 0, st>>>(w.RA, rows_ra, L, w.ras);
+      else
+        channel_sum_kernel<R><<<(unsigned)((rows_ra * 32 + 255) / 256), 256, 0, st>>>(
+            w.RA, nullptr, 1, rows_ra, L, w.ras);
       CK_LAUNCH(h);
       const long long rows_pt = (long long)n * Kmax;
       channel_sum_kernel<R><<<(unsigned)((rows_pt * 32 + 255) / 256), 256, 0, st>>>(

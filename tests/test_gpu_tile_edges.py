@@ -50,4 +50,4 @@ def test_tile_edges_match_oracle(gpu_lib, coeff_dir, sensor, channels, profiles,
     seed = rng.normal(size=rts.radiance.shape)
     ad, _ = h.adjoint(atm, sfc, geo, opt, seed)
     kt = np.einsum("pl,plk->pk", seed, km.temperature)
-    assert _rel(ad["temperature"], kt) < 1e-5 if precision else 1e-10
+    assert _rel(ad["temperature"], kt) < (1e-5 if precision else 1e-10)
