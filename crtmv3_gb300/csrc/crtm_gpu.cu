@@ -837,11 +837,11 @@ struct Work {
 };
 
 template <int G, class R> struct Tune;
-template <> struct Tune<1, double> { static constexpr int FWD = 4, AD = 2; };
+template <> struct Tune<1, double> { static constexpr int FWD = 4, AD = 1; };
 template <> struct Tune<1, float> { static constexpr int FWD = 8, AD = 4; };
-template <> struct Tune<2, double> { static constexpr int FWD = 4, AD = 2; };
+template <> struct Tune<2, double> { static constexpr int FWD = 4, AD = 1; };
 template <> struct Tune<2, float> { static constexpr int FWD = 8, AD = 4; };
-template <> struct Tune<3, double> { static constexpr int FWD = 4, AD = 4; };
+template <> struct Tune<3, double> { static constexpr int FWD = 4, AD = 1; };
 template <> struct Tune<3, float> { static constexpr int FWD = 8, AD = 8; };
 // profiles per absorb_ad CTA
 template <int G, class R> constexpr int ad_profiles() { return Tune<G, R>::AD * AD_WARPS; }
@@ -1398,13 +1398,13 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
     }
     {
       StageScope sc(h, 3, st);
-      dim3 ga((L + 31) / 32, (n + ad_profiles<G, R>() - 1) / ad_profiles<G, R>());
-      if (ho_only)
-        absorb_ad_kernel<G, R, NPA, 1><<<ga, 32 * AD_WARPS, 0, st>>>(
-            K, L, s.Lp, n, s.d_C, s.d_cmask, w.pv.Dg, s.tables.pdp, w.OD, w.SC, oa, w.RA);
-      else
-        absorb_ad_kernel<G, R, NPA, 0><<<ga, 32 * AD_WARPS, 0, st>>>(
-            K, L, s.Lp, n, s.d_C, s.d_cmask, w.pv.Dg, s.tables.pdp, w.OD, w.SC, oa, w.RA);
+      const int tiles = (L + 31) / 32, wp = ad_warps(tiles, n, NPA);
+      const dim3 ga(tiles, (n + wp * NPA - 1) / (wp * NPA));
+      const size_t ad_smem = ad_smem_bytes<G, R, NPA>(wp);
+      const auto ad = wp == 1 ? (ho_only ? absorb_ad_kernel<G, R, NPA, 1, 1> : absorb_ad_kernel<G, R, NPA, 0, 1>)
+                              : (ho_only ? absorb_ad_kernel<G, R, NPA, 1, AD_WARPS> : absorb_ad_kernel<G, R, NPA, 0, AD_WARPS>);
+      if (reserve_smem(h, ad, ad_smem, "absorb_ad")) return CRTM_GPU_FAILURE;
+      ad<<<ga, 32 * wp, ad_smem, st>>>(K, L, s.Lp, n, s.d_C, s.d_cmask, w.pv.Dg, s.tables.pdp, w.OD, w.SC, oa, w.RA);
       CK_LAUNCH(h);
       if (s.ov.n > 0) {   // the OPTRAN terms' temperature and water vapour adjoints
         int h2o_out = -1;

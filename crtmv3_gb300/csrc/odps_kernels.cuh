@@ -189,6 +189,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
 }
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
@@ -202,14 +206,23 @@ __device__ __forceinline__ double widen(float f) {
   return m == 0u ? __hiloint2double((int)u, 0) : double(f);
 }
 __device__ __forceinline__ double widen(double d) { return d; }
+
 // Coefficient tile of one reference layer: NS slots x 32 channels starting at
-// channel l0 of C[k][s][Lp] (Lp a multiple of 32, rows 128-byte aligned).
-template <int NS>
-__device__ __forceinline__ void load_c_tile(float (*dst)[32], const float* __restrict__ C, int k,
+// channel l0 of C[k][s][Lp] (Lp a multiple of 32, rows 128-byte aligned);
+// widened on the way where R is double.
+template <int NS, class R>
+__device__ __forceinline__ void load_c_tile(R (*dst)[32], const float* __restrict__ C, int k,
                                             int Lp, int l0, int tid, int nthreads) {
   for (int i = tid; i < NS * 8; i += nthreads) {
     const int s = i >> 3, q = i & 7;
-    cp_async16(&dst[s][q * 4], C + ((size_t)k * NS + s) * Lp + l0 + q * 4, 16);
+    const float* src = C + ((size_t)k * NS + s) * Lp + l0 + q * 4;
+    if constexpr (sizeof(R) == 4) {
+      cp_async16(&dst[s][q * 4], src, 16);
+    } else {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+      R* d = &dst[s][q * 4];
+      d[0] = widen(v.x); d[1] = widen(v.y); d[2] = widen(v.z); d[3] = widen(v.w);
+    }
   }
 }
 
@@ -676,7 +689,7 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) absorb_fwd_kernel(int K, int k
       } else {
         const float4 v = l < Lp ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
         R* d = &cs[buf][s][q * 4];
-        d[0] = to_f64(v.x); d[1] = to_f64(v.y); d[2] = to_f64(v.z); d[3] = to_f64(v.w);
+        d[0] = widen(v.x); d[1] = widen(v.y); d[2] = widen(v.z); d[3] = widen(v.w);
       }
     }
     if (live > 0) {
@@ -1587,8 +1600,15 @@ __global__ void __launch_bounds__(128) column_finish_kernel(ColumnArgs<R> a) {
 // ---------------------------------------------------------------------------
 // 4. absorption adjoint: reference-layer adjoints RA[p][v][k][l], v = 0 the
 //    temperature, v = 1+j the j-th requested absorber.  CTA = 32 channels
-//    (lanes) x 4 warps, each warp NP profiles; the coefficient slice of layer k
-//    for the CTA's channels is staged in shared memory and used by all warps.
+//    (lanes) x up to 4 warps, each warp NP profiles; the coefficient slice of
+//    layer k for the CTA's channels is staged in shared memory and used by all
+//    warps.
+//
+//    Bound: FP32 issue and shared-memory reads in the mixed form, FP64 issue in
+//    the FP64 form.  There a coefficient is widened once per CTA, by integer
+//    instructions, and a warp holds one profile: widening each coefficient per
+//    pair of profiles took a third of the pipe, and small batches spread over
+//    twice the schedulers.
 // ---------------------------------------------------------------------------
 struct OutAbs {
   int n;                  // requested absorber adjoints
@@ -1596,6 +1616,16 @@ struct OutAbs {
 };
 
 constexpr int AD_WARPS = 4;
+
+// Warps per CTA: 4, which share a coefficient tile, or 1 where 4 would leave
+// SMs without a CTA.
+inline int ad_warps(int tiles, int n, int np) {
+  return (long long)tiles * ((n + AD_WARPS * np - 1) / (AD_WARPS * np)) < 152 * 2 ? 1 : AD_WARPS;
+}
+template <int G, class R, int NP>
+inline size_t ad_smem_bytes(int warps) {
+  return sizeof(R) * 2 * ((size_t)Group<G>::NS * 32 + (size_t)warps * DLayout<G>::NX * NP);
+}
 
 // OUTSET 0: adjoints of every ODPS absorber; 1: only absorbers 0 and 1 (H2O and,
 // for groups 1-2, O3), which skips the partials the other absorbers' own
@@ -1609,20 +1639,23 @@ __host__ __device__ constexpr bool q_needed(int q) {
   return true;
 }
 
-template <int G, class R, int NP, int OUTSET>
-__global__ void __launch_bounds__(32 * AD_WARPS) absorb_ad_kernel(
+template <int G, class R, int NP, int OUTSET, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) absorb_ad_kernel(
     int K, int L, int Lp, int n_chunk, const float* __restrict__ C,
     const unsigned* __restrict__ cmask, const R* __restrict__ Dg,
     const double* __restrict__ pdp_tab, const R* __restrict__ ODAD, const R* __restrict__ SC,
     OutAbs oa, R* __restrict__ RA) {
   constexpr int NS = Group<G>::NS, JM = Group<G>::JM, NV = Group<G>::NV;
   constexpr int NNZ = DLayout<G>::NNZ, NX = DLayout<G>::NX;
-  constexpr int DCH = NX * NP * (int)sizeof(R) / 16;   // 16-byte chunks of one warp's D slice
-  __shared__ __align__(16) float cs[2][NS][32];
-  __shared__ __align__(16) R ds[2][AD_WARPS][NX * NP];
+  // one warp's D slice in 16-byte chunks (8-byte ones where it is an odd number of doubles)
+  constexpr int DCB = NX * NP * (int)sizeof(R) % 16 == 0 ? 16 : 8;
+  constexpr int DCH = NX * NP * (int)sizeof(R) / DCB;
+  extern __shared__ __align__(16) unsigned char ad_smem[];
+  auto cs = reinterpret_cast<R (*)[NS][32]>(ad_smem);                  // [2][NS][32]
+  R* ds = reinterpret_cast<R*>(ad_smem) + 2 * NS * 32;                 // [2][warps][NX * NP]
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int l0 = blockIdx.x * 32, l = l0 + lane;
-  const int pg = blockIdx.y * AD_WARPS + wib;
+  const int pg = blockIdx.y * WARPS + wib;
   const int p0 = pg * NP;
   const bool active = l < L;
   const unsigned wmask = __reduce_or_sync(FULL, active ? cmask[l] : 0u);
@@ -1641,10 +1674,16 @@ __global__ void __launch_bounds__(32 * AD_WARPS) absorb_ad_kernel(
     for (int a = 0; a < JM; a++) Sgazp[p][a] = Sgatzp[p][a] = R(0);
   }
   auto stage = [&](int k, int buf) {
-    load_c_tile<NS>(cs[buf], C, k, Lp, l0, threadIdx.x, 32 * AD_WARPS);
+    load_c_tile<NS, R>(cs[buf], C, k, Lp, l0, threadIdx.x, 32 * WARPS);
     if (group_ok) {
       const R* src = Db + (size_t)k * NX * NP;
-      for (int i = lane; i < DCH; i += 32) cp_async16(&ds[buf][wib][i * (16 / sizeof(R))], src + i * (16 / sizeof(R)), 16);
+      R* dst = ds + (size_t)(buf * WARPS + wib) * (NX * NP);
+      for (int i = lane; i < DCH; i += 32) {
+        if constexpr (DCB == 16)
+          cp_async16(dst + i * (16 / sizeof(R)), src + i * (16 / sizeof(R)), 16);
+        else
+          cp_async8(dst + i * (8 / sizeof(R)), src + i * (8 / sizeof(R)));
+      }
     }
     cp_async_commit();
   };
@@ -1665,8 +1704,8 @@ __global__ void __launch_bounds__(32 * AD_WARPS) absorb_ad_kernel(
       odc[p] = odn[p];
       if (k > 0 && active && p0 + p < n_chunk) odn[p] = ODAD[((size_t)(p0 + p) * K + (k - 1)) * L + l];
     }
-    const float (*ct)[32] = cs[k & 1];
-    const R* Dk = ds[k & 1][wib];
+    const R (*ct)[32] = cs[k & 1];
+    const R* Dk = ds + (size_t)((k & 1) * WARPS + wib) * (NX * NP);
     R E[NP][NV];
 #pragma unroll
     for (int p = 0; p < NP; p++)
@@ -1678,7 +1717,7 @@ __global__ void __launch_bounds__(32 * AD_WARPS) absorb_ad_kernel(
       constexpr int j = slot_component<G>(s);
       if constexpr (!q_needed<G, OUTSET>(q)) return;
       if (!(wmask & (1u << j))) return;
-      const R c = R(ct[s][lane]);
+      const R c = ct[s][lane];
 #pragma unroll
       for (int p = 0; p < NP; p++) E[p][q] += c * Dk[e * NP + p];
     });
@@ -1750,7 +1789,6 @@ inline size_t map_smem_bytes(int K, int Kmax, int nv, int ct) {
                       (size_t)Kmax * MAX_UBAND) +
          sizeof(int) * 2 * (size_t)Kmax + 16;
 }
-
 template <class R>
 __global__ void __launch_bounds__(256) map_kernel(MapArgs<R> m) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
