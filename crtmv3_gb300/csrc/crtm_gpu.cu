@@ -1903,10 +1903,15 @@ struct TLArgs {
   double* bt_tl;
 };
 
-// One warp per (profile, TL_CH consecutive channels), lanes over the layers:
-// each perturbation value is loaded once for the warp's channels, whose
-// TL_CH sums are independent accumulations (the same order per channel as a
-// warp per channel would take).
+// One warp per (profile, TL_CH consecutive channels), lanes over a block's rows
+// and layers: each perturbation value is loaded once for the warp's channels.
+//
+// Bound: the FP64 pipe (a multiply-add per stored Jacobian value, 2 per clock
+// and SM), above the HBM read.  So a profile that fills its layer stride runs
+// over rows x layers as one index (101 layers a row leave the fourth 32 lanes
+// nearly empty, a quarter of the multiply-adds), and the 8 channels' sums over
+// the lanes take 9 additions instead of 40: a step of the exchange adds one
+// half of the channels' sums and hands over the other.
 constexpr int TL_CH = 8;
 
 __global__ void tl_kernel(TLArgs a) {
@@ -1917,6 +1922,7 @@ __global__ void tl_kernel(TLArgs a) {
   const int p = (int)(w / groups), l0 = (int)(w % groups) * TL_CH;
   const int nch = min(TL_CH, a.L - l0);
   const int Ku = a.n_layers[p];
+  const bool whole = Ku == a.Km;   // no padded layers: a block's rows in one run
   double s[TL_CH];
 #pragma unroll
   for (int c = 0; c < TL_CH; c++) s[c] = 0.0;
@@ -1927,12 +1933,14 @@ __global__ void tl_kernel(TLArgs a) {
     for (int r = 0; r < nrow; r++) {
       const double* dr = D + ((size_t)p * nrow + r) * a.Km;
       const double* kr = k0 + (size_t)r * a.Km;
-      for (int k = lane; k < Ku; k += 32) {
+      const int len = whole ? nrow * a.Km : Ku;
+      for (int k = lane; k < len; k += 32) {
         const double d = dr[k];
 #pragma unroll
         for (int c = 0; c < TL_CH; c++)
           if (c < nch) s[c] += kr[c * cstride + k] * d;
       }
+      if (whole) break;
     }
   };
   rows(a.kt, a.d.temperature, 1);
@@ -1944,13 +1952,18 @@ __global__ void tl_kernel(TLArgs a) {
   rows(a.kar, a.d.aerosol_effective_radius, a.NA);
   rows(a.kav, a.d.aerosol_effective_variance, a.NA);
   rows(a.krh, a.d.relative_humidity, 1);
-  double mine = 0.0;
+  // channel c's sum ends on the lanes whose low three bits are c
 #pragma unroll
-  for (int c = 0; c < TL_CH; c++) {
-    double v = s[c];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == c) mine = v;
+  for (int h = TL_CH / 2; h > 0; h >>= 1) {
+    const bool up = lane & h;
+#pragma unroll
+    for (int c = 0; c < h; c++) {
+      const double give = up ? s[c] : s[c + h], keep = up ? s[c + h] : s[c];
+      s[c] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+    }
   }
+  double mine = s[0];
+  for (int o = TL_CH; o < 32; o <<= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
   if (lane >= nch) return;
   const size_t pl = (size_t)p * a.L + l0 + lane;
   double t = mine;
@@ -2066,21 +2079,56 @@ int tl_apply(crtm_gpu_handle h, const crtm_gpu_tl_in* tl, double* bt_tl, cudaStr
 }
 
 // out[p][j] = sum_l w[p][l] K[p][l][j] (j over a block's rows x layers), zero
-// for profiles whose trajectory status is not 0: one thread per (p, j), the
-// channels' rows read coalesced across j.
-__global__ void channel_contract_kernel(const double* __restrict__ K, int P, int L, int rowlen,
-                                        const double* __restrict__ w, const int* __restrict__ status,
-                                        double* __restrict__ out) {
-  const int p = blockIdx.y;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P || j >= rowlen) return;
+// for profiles whose trajectory status is not 0, for every block of the
+// trajectory in one launch: a CTA takes 64 values of j of one profile and
+// block, its four quarters every fourth channel.
+//
+// Bound: the FP64 pipe, above the HBM read (as tl_kernel).  With a thread per
+// (profile, j) walking all channels and a launch per block, blocks of one value
+// a channel (surface terms) ran 616 dependent steps on one lane per profile:
+// 72 us each for 300 profiles.
+struct ContractArgs {
+  static constexpr int MAX = 14;
+  const double* k[MAX];
+  double* out[MAX];
+  int rowlen[MAX], chunk0[MAX + 1];   // first chunk of each block
+  int n, L;
+  const double* w;
+  const int* status;
+};
+constexpr int CONTRACT_COLS = 64, CONTRACT_THREADS = 256;
+
+__global__ void __launch_bounds__(CONTRACT_THREADS) channel_contract_kernel(ContractArgs a) {
+  __shared__ double part[CONTRACT_THREADS];
+  const int p = blockIdx.y, tid = threadIdx.x, L = a.L;
+  int f = 0;
+  while (f + 1 < a.n && (int)blockIdx.x >= a.chunk0[f + 1]) f++;
+  const int rowlen = a.rowlen[f];
+  const bool scalar = rowlen == 1;   // one value a channel: all threads over the channels
+  const int j = scalar ? 0 : ((int)blockIdx.x - a.chunk0[f]) * CONTRACT_COLS + (tid & (CONTRACT_COLS - 1));
+  const int l0 = scalar ? tid : tid / CONTRACT_COLS;
+  const int step = scalar ? CONTRACT_THREADS : CONTRACT_THREADS / CONTRACT_COLS;
   double acc = 0.0;
-  if (!status[p]) {
-    const double* kp = K + (size_t)p * L * rowlen + j;
-    const double* wp = w + (size_t)p * L;
-    for (int l = 0; l < L; l++) acc += wp[l] * kp[(size_t)l * rowlen];
+  if (j < rowlen && !a.status[p]) {
+    const double* kp = a.k[f] + (size_t)p * L * rowlen + j;
+    const double* wp = a.w + (size_t)p * L;
+#pragma unroll 8
+    for (int l = l0; l < L; l += step) acc += wp[l] * kp[(size_t)l * rowlen];
   }
-  out[(size_t)p * rowlen + j] = acc;
+  part[tid] = acc;
+  __syncthreads();
+  double* out = a.out[f] + (size_t)p * rowlen;
+  if (scalar) {
+    for (int o = CONTRACT_THREADS / 2; o > 0; o >>= 1) {
+      if (tid < o) part[tid] += part[tid + o];
+      __syncthreads();
+    }
+    if (tid == 0) out[0] = part[0];
+  } else if (tid < CONTRACT_COLS && j < rowlen) {
+    double v = part[tid];
+    for (int q = CONTRACT_COLS; q < CONTRACT_THREADS; q += CONTRACT_COLS) v += part[tid + q];
+    out[j] = v;
+  }
 }
 
 // The adjoint about the stored trajectory: the outputs of CRTM_Adjoint for
@@ -2112,6 +2160,8 @@ int ad_apply(crtm_gpu_handle h, const double* bt_ad, crtm_gpu_adjoint_out* ad, c
       {g.k.relative_humidity, ad->relative_humidity, Km, "relative humidity"},
       {g.k.wind_speed, ad->wind_speed, 1, "wind speed"},
   };
+  ContractArgs ca{};
+  ca.L = g.L; ca.w = bt_ad; ca.status = g.status;
   for (const Block& x : blocks) {
     if (!x.out) continue;
     if (!x.k) return fail(h, "the trajectory holds no %s Jacobian", x.what);
@@ -2121,8 +2171,14 @@ int ad_apply(crtm_gpu_handle h, const double* bt_ad, crtm_gpu_adjoint_out* ad, c
         return fail(h, "cudaMemsetAsync failed");
       continue;
     }
-    const dim3 grid((unsigned)((x.rowlen + 127) / 128), (unsigned)g.P);
-    channel_contract_kernel<<<grid, 128, 0, st>>>(x.k, g.P, g.L, x.rowlen, bt_ad, g.status, x.out);
+    ca.k[ca.n] = x.k;
+    ca.out[ca.n] = x.out;
+    ca.rowlen[ca.n] = x.rowlen;
+    ca.chunk0[ca.n + 1] = ca.chunk0[ca.n] + (x.rowlen + CONTRACT_COLS - 1) / CONTRACT_COLS;
+    ca.n++;
+  }
+  if (ca.n > 0) {
+    channel_contract_kernel<<<dim3((unsigned)ca.chunk0[ca.n], (unsigned)g.P), CONTRACT_THREADS, 0, st>>>(ca);
     CK_LAUNCH(h);
   }
   mark_done(h, st);
