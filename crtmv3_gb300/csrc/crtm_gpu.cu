@@ -140,6 +140,7 @@ struct Sensor {
   unsigned* d_cmask = nullptr;   // [L]
   double* d_tab = nullptr;       // concatenated tables
   double* d_spec = nullptr;      // c1,c2,b1,b2,cbr,frequency,wavenumber [7][L]
+  int* d_out = nullptr;          // [L] caller's column of each device channel (SpecView::out)
   SensorTables tables{};
   RefSums refsums{};
   SpecView spec{};
@@ -154,6 +155,7 @@ struct Sensor {
   // (crtm_gpu_set_channel_subset): L and the device arrays above hold the
   // processed channels only
   int L_all = 0, Lp_all = 0;
+  std::vector<int> order;            // [L] device channel -> the caller's
   std::vector<float> C_all;          // [K][NS][Lp_all]
   std::vector<unsigned> cmask_all;   // [L_all]
   std::vector<double> spec_all;      // [7][L_all]
@@ -182,8 +184,8 @@ bool upload_optran(Sensor& s, const std::vector<int>& pos, std::string& err) {
   std::vector<double> cf;
   const int n = pos.empty() ? s.L_all : (int)pos.size();
   const size_t nc = (size_t)OPT_NU * (OPT_ORDER + 1);
-  for (int l = 0; l < n; l++) {
-    const int q = pos.empty() ? l : pos[l];
+  for (int l = 0; l < n; l++) {   // device channels
+    const int q = pos.empty() ? s.order[l] : pos[s.order[l]];
     if (q < 0 || q >= (int)s.o_n.size() || s.o_n[q] <= 0) continue;
     ch.push_back(l);
     ix.insert(ix.end(), s.o_idx.begin() + (size_t)q * 8, s.o_idx.begin() + (size_t)q * 8 + 8);
@@ -204,6 +206,8 @@ bool upload_optran(Sensor& s, const std::vector<int>& pos, std::string& err) {
   s.ov.ch = s.d_och; s.ov.idx = s.d_oidx; s.ov.coef = s.d_ocoef;
   return true;
 }
+
+bool upload_channels(Sensor& s, const std::vector<int>& pos, std::string& err);
 
 bool load_sensor(const std::string& dir, const std::string& id, Sensor& s, std::string& err) {
   s.id = id;
@@ -399,14 +403,8 @@ bool load_sensor(const std::string& dir, const std::string& id, Sensor& s, std::
   s.cmask_all = cmask;
   s.spec_all = spec;
   cudaError_t ce;
-  if ((ce = cudaMalloc(&s.d_C, Cd.size() * sizeof(float))) != cudaSuccess ||
-      (ce = cudaMalloc(&s.d_cmask, cmask.size() * sizeof(unsigned))) != cudaSuccess ||
-      (ce = cudaMalloc(&s.d_tab, tab.size() * sizeof(double))) != cudaSuccess ||
-      (ce = cudaMalloc(&s.d_spec, spec.size() * sizeof(double))) != cudaSuccess ||
-      (ce = cudaMemcpy(s.d_C, Cd.data(), Cd.size() * sizeof(float), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (ce = cudaMemcpy(s.d_cmask, cmask.data(), cmask.size() * sizeof(unsigned), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (ce = cudaMemcpy(s.d_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (ce = cudaMemcpy(s.d_spec, spec.data(), spec.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess) {
+  if ((ce = cudaMalloc(&s.d_tab, tab.size() * sizeof(double))) != cudaSuccess ||
+      (ce = cudaMemcpy(s.d_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess) {
     err = std::string("device upload of ") + id + " coefficients failed: " + cudaGetErrorString(ce);
     return false;
   }
@@ -417,13 +415,9 @@ bool load_sensor(const std::string& dir, const std::string& id, Sensor& s, std::
   t.ref_t = s.d_tab + o_t; t.ref_a = s.d_tab + o_a; t.min_a = s.d_tab + o_mn; t.max_a = s.d_tab + o_mx;
   t.pdp = s.d_tab + o_pdp; t.zgeo = s.d_tab + o_z; t.ref_p = s.d_tab + o_rp;
   t.o_alpha = s.o_alpha; t.o_c1 = s.o_c1; t.o_c2 = s.o_c2;
-  if (!upload_optran(s, std::vector<int>(), err)) return false;
   s.refsums.tz_ref = s.d_tab + o_tzr; s.refsums.tzp_ref = s.d_tab + o_tzpr;
   s.refsums.gazp_ref = s.d_tab + o_gzr; s.refsums.gatzp_ref = s.d_tab + o_gtr;
-  s.spec.c1 = s.d_spec; s.spec.c2 = s.d_spec + L; s.spec.b1 = s.d_spec + 2 * L;
-  s.spec.b2 = s.d_spec + 3 * L; s.spec.cbr = s.d_spec + 4 * L;
-  s.spec.freq = s.d_spec + 5 * L; s.spec.wn = s.d_spec + 6 * L;
-  return true;
+  return upload_channels(s, std::vector<int>(), err);
 }
 
 // The device arrays of the channels at file positions `pos` (all channels
@@ -437,44 +431,58 @@ bool upload_channels(Sensor& s, const std::vector<int>& pos, std::string& err) {
   std::vector<float> Cd((size_t)K * NS * Lp, 0.0f);
   std::vector<unsigned> cmask(std::max(L, 1), 0u);
   std::vector<double> spec((size_t)7 * std::max(L, 1), 0.0);
+  // device order: by the channels' absorption components, along a Gray code of
+  // their sets, so that a tile's channels have few components between them
+  // (the absorption kernels walk the union)
+  s.order.resize(L);
+  for (int l = 0; l < L; l++) s.order[l] = l;
+  const auto rank = [&](int l) {
+    unsigned m = s.cmask_all[all ? l : pos[l]];
+    for (int sh = 1; sh < 32; sh <<= 1) m ^= m >> sh;
+    return m;
+  };
+  std::stable_sort(s.order.begin(), s.order.end(), [&](int x, int y) { return rank(x) < rank(y); });
+  std::vector<int> from(L);   // file position of each device channel
   for (int l = 0; l < L; l++) {
-    const int q = all ? l : pos[l];
-    for (size_t r = 0; r < (size_t)K * NS; r++) Cd[r * Lp + l] = s.C_all[r * s.Lp_all + q];
+    const int q = all ? s.order[l] : pos[s.order[l]];
+    from[l] = q;
     cmask[l] = s.cmask_all[q];
     for (int f = 0; f < 7; f++) spec[(size_t)f * L + l] = s.spec_all[(size_t)f * s.L_all + q];
   }
+  for (size_t r = 0; r < (size_t)K * NS; r++)
+    for (int l = 0; l < L; l++) Cd[r * Lp + l] = s.C_all[r * s.Lp_all + from[l]];
   float* dC = nullptr;
   unsigned* dm = nullptr;
   double* ds = nullptr;
+  int* dord = nullptr;
   cudaError_t ce;
   if ((ce = cudaMalloc(&dC, Cd.size() * sizeof(float))) != cudaSuccess ||
       (ce = cudaMalloc(&dm, cmask.size() * sizeof(unsigned))) != cudaSuccess ||
       (ce = cudaMalloc(&ds, spec.size() * sizeof(double))) != cudaSuccess ||
+      (ce = cudaMalloc(&dord, std::max(L, 1) * sizeof(int))) != cudaSuccess ||
+      (ce = cudaMemcpy(dord, s.order.data(), L * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (ce = cudaMemcpy(dC, Cd.data(), Cd.size() * sizeof(float), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (ce = cudaMemcpy(dm, cmask.data(), cmask.size() * sizeof(unsigned), cudaMemcpyHostToDevice)) != cudaSuccess ||
       (ce = cudaMemcpy(ds, spec.data(), spec.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess) {
-    cudaFree(dC); cudaFree(dm); cudaFree(ds);
+    cudaFree(dC); cudaFree(dm); cudaFree(ds); cudaFree(dord);
     err = std::string("device upload of the channel subset failed: ") + cudaGetErrorString(ce);
     return false;
   }
-  cudaFree(s.d_C); cudaFree(s.d_cmask); cudaFree(s.d_spec);
-  s.d_C = dC; s.d_cmask = dm; s.d_spec = ds;
+  cudaFree(s.d_C); cudaFree(s.d_cmask); cudaFree(s.d_spec); cudaFree(s.d_out);
+  s.d_C = dC; s.d_cmask = dm; s.d_spec = ds; s.d_out = dord;
   s.L = L; s.Lp = Lp; s.tables.L = L;
   s.spec.c1 = ds; s.spec.c2 = ds + L; s.spec.b1 = ds + 2 * L;
   s.spec.b2 = ds + 3 * L; s.spec.cbr = ds + 4 * L;
   s.spec.freq = ds + 5 * L; s.spec.wn = ds + 6 * L;
-  for (int f = 0; f < 7; f++) {
-    std::vector<double>* v[7] = {&s.c1, &s.c2, &s.b1, &s.b2, &s.cbr, &s.freq, &s.wn};
-    v[f]->assign(spec.begin() + (size_t)f * L, spec.begin() + (size_t)f * L + L);
-  }
+  s.spec.out = dord;
   s.processed = pos;
   return upload_optran(s, pos, err);
 }
 
 void free_sensor(Sensor& s) {
-  cudaFree(s.d_C); cudaFree(s.d_cmask); cudaFree(s.d_tab); cudaFree(s.d_spec);
+  cudaFree(s.d_C); cudaFree(s.d_cmask); cudaFree(s.d_tab); cudaFree(s.d_spec); cudaFree(s.d_out);
   cudaFree(s.d_oidx); cudaFree(s.d_och); cudaFree(s.d_ocoef); cudaFree(s.d_zc);
-  s.d_C = nullptr; s.d_cmask = nullptr; s.d_tab = nullptr; s.d_spec = nullptr;
+  s.d_C = nullptr; s.d_cmask = nullptr; s.d_tab = nullptr; s.d_spec = nullptr; s.d_out = nullptr;
   s.d_oidx = nullptr; s.d_och = nullptr; s.d_ocoef = nullptr; s.d_zc = nullptr;
 }
 
@@ -1024,8 +1032,8 @@ struct SfcModel {
 // Profiles whose water coverage is not 1 raise error 13 (the land, snow and
 // ice models are not built).
 __global__ void irwater_kernel(IRWaterLut W, int P, int L, const double* wn, const double* zenith,
-                               const double* t_water, const double* water_cov, const double* wind, double* E,
-                               double* EV, double* ET, int* error) {
+                               const double* t_water, const double* water_cov, const double* wind,
+                               const int* out, double* E, double* EV, double* ET, int* error) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)P * L) return;
   const int p = (int)(i / L), l = (int)(i % L);
@@ -1034,9 +1042,10 @@ __global__ void irwater_kernel(IRWaterLut W, int P, int L, const double* wn, con
   v.d[0] = 1.0;
   t.d[1] = 1.0;
   const Dual<2> e = irssem<Dual<2>>(W, t, v, wn[l], zenith[p]);
-  E[i] = e.v;
-  EV[i] = e.d[0];
-  ET[i] = e.d[1];
+  const size_t pl = (size_t)p * L + out[l];
+  E[pl] = e.v;
+  EV[pl] = e.d[0];
+  ET[pl] = e.d[1];
 }
 
 int copy_chunk(crtm_gpu_handle h, const HostCopy* hc, int p0, int n, cudaStream_t st) {
@@ -1353,7 +1362,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
             if (mode == 1) {
               dim3 gt((L + 31) / 32, (Kmax + 31) / 32, std::min(n * o.ns, 65535));
               species_k_out_kernel<<<gt, dim3(32, 8), 0, st>>>(o.X, o.S, o.s0, o.ns, Kmax, L, p0, n, o.o,
-                                                               perm);
+                                                               perm, s.spec.out);
             } else {
               const long long rows = (long long)n * o.ns * Kmax;
               species_ad_out_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(o.X, o.S, o.s0, o.ns, Kmax, L,
@@ -1418,7 +1427,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
     if (mode == 1) {
       MapArgs<R> ma{};
       ma.K = K; ma.L = L; ma.Kmax = Kmax; ma.p_begin = p0; ma.n_chunk = n; ma.nv = nv; ma.ct = map_ct;
-      ma.b = bv; ma.pv = w.pv; ma.RA = w.RA; ma.PT = w.PT; ma.SC = w.SC;
+      ma.b = bv; ma.pv = w.pv; ma.RA = w.RA; ma.PT = w.PT; ma.SC = w.SC; ma.out = s.spec.out;
       ma.kt = kk->temperature; ma.ka = kk->absorber;
       StageScope sc(h, 4, st);
       dim3 gm((L + map_ct - 1) / map_ct, n);
@@ -1550,7 +1559,7 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
     if (cudaMemsetAsync(h->d_error, 0, sizeof(int), st) != cudaSuccess) return fail(h, "error flag reset failed");
     irwater_kernel<<<(unsigned)((PL + 255) / 256), 256, 0, st>>>(h->irw, b->n_profiles, s.L, s.spec.wn,
                                                                  b->sensor_zenith_angle, b->water_temperature,
-                                                                 b->water_coverage, b->wind_speed, E, E + PL,
+                                                                 b->water_coverage, b->wind_speed, s.spec.out, E, E + PL,
                                                                  E + 2 * PL, h->d_error);
     CK_LAUNCH(h);
     bm = *b;

@@ -271,6 +271,10 @@ CRTM_HD void zero_row(double* o, size_t pl, int Kmax, int from) {
 struct SpecView {
   const double* c1, *c2, *b1, *b2, *cbr;
   const double* freq, *wn;   // GHz, cm^-1
+  // the caller's column of each channel: a sensor's tables and every
+  // intermediate hold the channels ordered by the absorption components they
+  // have, so that the channels of a tile share them
+  const int* out;
 };
 
 // Running sums of the reference profile (the *_ref terms of ODPS_Predictor.f90:707-759).
@@ -845,7 +849,7 @@ __global__ void __launch_bounds__(128) column_kernel(ColumnArgs<R> a) {
   };
   if (st != 0) {
     if (l < L) {
-      const size_t pl = (size_t)gp * L + l;
+      const size_t pl = (size_t)gp * L + a.sp.out[l];
       a.radiance[pl] = 0.0;
       a.bt[pl] = 0.0;
       ext_scalars(pl, 0.0, 0.0, 0.0, 0.0);
@@ -877,7 +881,7 @@ __global__ void __launch_bounds__(128) column_kernel(ColumnArgs<R> a) {
   }
   __syncthreads();
   if (l >= L) return;
-  const size_t pl = (size_t)gp * L + l;
+  const size_t pl = (size_t)gp * L + a.sp.out[l];
   const double* sc = a.pv.scal + (size_t)p * PREP_SCAL;
   const R inv_sec = R(sc[2]);
   const R inv_u = R(sc[3]);
@@ -1178,7 +1182,7 @@ __global__ void __launch_bounds__(COL_THREADS) column_tile_kernel(ColumnArgs<R> 
   const RtsExt x = EXT ? a.x : RtsExt{};
   if (st != 0) {   // column_finish_kernel writes the profile's zeros
     if (tid < cw && l < L) {
-      const size_t pl = (size_t)gp * L + l;
+      const size_t pl = (size_t)gp * L + a.sp.out[l];
       zero_row(x.lod, pl, Kmax, 0);
       zero_row(x.upw, pl, Kmax, 0);
       zero_row(x.ovc, pl, Kmax, 0);
@@ -1211,7 +1215,7 @@ __global__ void __launch_bounds__(COL_THREADS) column_tile_kernel(ColumnArgs<R> 
   int* ihis = ilos + (K + 1);
   unsigned* flags = reinterpret_cast<unsigned*>(ihis + (K + 1));   // [ceil(K/32)][cw] clamped layers
   const bool chan = l < L;
-  const size_t pl = (size_t)gp * L + (chan ? l : 0);
+  const size_t pl = (size_t)gp * L + a.sp.out[chan ? l : 0];
   R* od = a.OD + (size_t)p * K * L + l;
   // ---- stage the tables and the reference optical depths
   {
@@ -1296,7 +1300,7 @@ __global__ void __launch_bounds__(COL_THREADS) column_tile_kernel(ColumnArgs<R> 
   // rows of the CTA's channels out of shared memory (v[ku][c]) to o[pl][Kmax], layers across lanes
   auto rows_out = [&](double* o, const R* v) {
     for (int cc = tid >> 5; cc < cw && l0 + cc < L; cc += COL_THREADS / 32) {
-      double* r = o + ((size_t)gp * L + l0 + cc) * Kmax;
+      double* r = o + ((size_t)gp * L + a.sp.out[l0 + cc]) * Kmax;
       for (int ku = tid & 31; ku < Kmax; ku += 32) r[ku] = ku < Ku && v ? double(v[ku * CS + cc]) : 0.0;
     }
   };
@@ -1483,7 +1487,7 @@ __global__ void __launch_bounds__(128) column_finish_kernel(ColumnArgs<R> a) {
   const int st = a.pv.status[p];
   if (l == 0 && a.status) a.status[gp] = st;
   if (l >= L) return;
-  const size_t pl = (size_t)gp * L + l;
+  const size_t pl = (size_t)gp * L + a.sp.out[l];
   const RtsExt x = EXT ? a.x : RtsExt{};
   auto ext_scalars = [&](double e, double up, double down, double bs) {
     if (x.emis) x.emis[pl] = e;
@@ -1779,6 +1783,7 @@ struct MapArgs {
   const R* RA;   // [n][nv][K][L]
   const R* PT;   // [n][Kmax][L]
   const R* SC;   // [n][L]
+  const int* out;   // SpecView::out
   double* kt;    // [P][L][Kmax]
   double* ka;    // [P][L][nv-1][Kmax]
 };
@@ -1841,7 +1846,7 @@ __global__ void __launch_bounds__(256) map_kernel(MapArgs<R> m) {
 #pragma unroll
     for (int i = 0; i < 4; i++) w[i] = i < n ? uws[i * Kmax + ku] : R(0);
     for (int c = wib; c < ncl; c += 8) {
-      const size_t pl = (size_t)gp * L + l0 + c;
+      const size_t pl = (size_t)gp * L + m.out[l0 + c];
       const R scl = sct[c];
       for (int v = 0; v < nv; v++) {
         double* out = v == 0 ? m.kt + pl * Kmax : m.ka + (pl * (nv - 1) + (v - 1)) * Kmax;

@@ -193,7 +193,7 @@ __device__ __forceinline__ CloudyColumn column_inputs(const ScatterArgs<R>& a, i
   c.microwave = a.microwave != 0;
   c.freq = a.microwave ? a.sp.freq[l] : a.sp.wn[l];
   c.mu_sensor = a.pv.scal[(size_t)p * PREP_SCAL + 1];
-  const size_t pl = (size_t)gp * a.L + l;
+  const size_t pl = (size_t)gp * a.L + a.sp.out[l];
   c.emissivity = a.b.emissivity[pl];
   c.c1 = a.sp.c1[l]; c.c2 = a.sp.c2[l]; c.b1 = a.sp.b1[l]; c.b2 = a.sp.b2[l];
   const double ts = a.b.land_cov[gp] * a.b.land_t[gp] + a.b.water_cov[gp] * a.b.water_t[gp] +
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_layers_kernel(Scatter
   const int kind = layer_optics<NZ, Rec, C>(c, a.lut, S, k, C(gas), C(c.temperature[k]), &od, Tm, Rm, src,
                                             NoSeed(), nullptr, a.x.sod ? &bs : nullptr);
   if (kind >= 0) {
-    const size_t pl = (size_t)gp * L + l;
+    const size_t pl = (size_t)gp * L + a.sp.out[l];
     if (a.x.lod) a.x.lod[pl * Kmax + k] = double(od);
     if (a.x.sod && bs > 0.0) atomicAdd(a.x.sod + pl, bs);
   }
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_adding_kernel(Scatter
   const int p = blockIdx.y, gp = batch_profile(a.b, a.p_begin + p);
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= L) return;
-  const size_t pl = (size_t)gp * L + l;
+  const size_t pl = (size_t)gp * L + a.sp.out[l];
   if (a.pv.status[p] != 0) {
     a.radiance[pl] = 0.0;
     a.bt[pl] = 0.0;
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_soi_kernel(ScatterArg
   if (l >= L || a.pv.status[p] != 0) return;
   const CloudyColumn c = column_inputs(a, p, gp, l);
   if ((c.n_clouds == 0 && c.n_aerosols == 0) || !c.soi) return;
-  const size_t pl = (size_t)gp * L + l;
+  const size_t pl = (size_t)gp * L + a.sp.out[l];
   double rad = 0.0, rad_clear = 0.0;
   int code = 0;
   StreamSet<NZ, double> S;
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_kmatrix_kernel(Scatte
   const CloudyColumn c = column_inputs(a, p, gp, l);
   if (c.n_clouds == 0 && c.n_aerosols == 0) return;   // clear: the column kernel's Emission adjoint
   if (c.soi) return;                                   // scatter_soi_k_kernel
-  if (a.x.nfs) a.x.nfs[(size_t)gp * L + l] = c.nleg + 2;
+  if (a.x.nfs) a.x.nfs[(size_t)gp * L + a.sp.out[l]] = c.nleg + 2;
   double rad = 0.0, e_b = 0.0, Bs_b = 0.0;
   StreamSet<NZ, double> S;
   int code = stream_set<NZ, double>(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, c_gauss, S);
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_soi_k_kernel(ScatterA
   if (l >= L || a.pv.status[p] != 0) return;
   const CloudyColumn c = column_inputs(a, p, gp, l);
   if ((c.n_clouds == 0 && c.n_aerosols == 0) || !c.soi) return;
-  if (a.x.nfs) a.x.nfs[(size_t)gp * L + l] = c.nleg + 2;
+  if (a.x.nfs) a.x.nfs[(size_t)gp * L + a.sp.out[l]] = c.nleg + 2;
   double rad = 0.0, e_b = 0.0, Bs_b = 0.0;
   StreamSet<NZ, double> S;
   int code = stream_set<NZ, double>(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, c_gauss, S);
@@ -797,9 +797,10 @@ __global__ void scatter_species_kernel(ScatterArgs<R> a) {
 }
 
 // K-matrix outputs of the species Jacobians: X[n][S][Kmax][L] slots s0..s0+ns-1
-// to out[P][L][ns][Kmax] (a shared-memory transpose of 32 x 32 tiles).
+// to out[P][L][ns][Kmax] (a shared-memory transpose of 32 x 32 tiles); chan:
+// SpecView::out.
 static __global__ void species_k_out_kernel(const double* X, int S, int s0, int ns, int Kmax, int L, int p_begin,
-                                     int n, double* out, const int* perm) {
+                                     int n, double* out, const int* perm, const int* chan) {
   __shared__ double tile[32][33];
   const int k0 = blockIdx.y * 32, l0 = blockIdx.x * 32;
   for (int ps = blockIdx.z; ps < n * ns; ps += gridDim.z) {
@@ -814,7 +815,7 @@ static __global__ void species_k_out_kernel(const double* X, int S, int s0, int 
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {
       const int l = l0 + i, k = k0 + threadIdx.x;
       const size_t gp = perm ? perm[p_begin + p] : p_begin + p;
-      if (l < L && k < Kmax) out[((gp * L + l) * ns + s) * Kmax + k] = tile[threadIdx.x][i];
+      if (l < L && k < Kmax) out[((gp * L + chan[l]) * ns + s) * Kmax + k] = tile[threadIdx.x][i];
     }
   }
 }
