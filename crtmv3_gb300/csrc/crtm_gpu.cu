@@ -1319,10 +1319,19 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
       if (split) {
         {
           StageScope sc(h, 7, st);
-          if (nz_max)
+          if constexpr (std::is_same<R, float>::value) {
+            if (soi) return fail(h, "internal: SOI K-matrix in the mixed form");
+            if (nz_max)
+              launch_adding_front<SC_NZ_MAX>(sa, ga, st);
+            else
+              launch_adding_front<5>(sa, ga, st);
+            CK_LAUNCH(h);
+            h->launches += launch_adding_team(sa, nz_max ? SC_NZ_MAX : 5, st) - 1;   // CK_LAUNCH counts one
+          } else if (nz_max) {
             launch_scatter_kmatrix<SC_NZ_MAX, R>(sa, ga, st, soi);
-          else
+          } else {
             launch_scatter_kmatrix<5, R>(sa, ga, st, soi);
+          }
           CK_LAUNCH(h);
         }
         {
@@ -1340,8 +1349,6 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
                 launch_scatter_contract<5, double>(sa, gl, st);
               CK_LAUNCH(h);
             }
-          } else if (soi) {
-            return fail(h, "internal: SOI K-matrix in the mixed form");
           }
         }
         {

@@ -17,11 +17,9 @@ void launch_scatter_layers_k(const ScatterArgs<R>& a, unsigned grid, cudaStream_
   scatter_layers_kernel<NZ, R, R, C><<<grid, SCATTER_THREADS, 0, st>>>(a, a.LBK);
 }
 
-template <int NZ, class R>
-void launch_scatter_kmatrix(const ScatterArgs<R>& a, dim3 grid, cudaStream_t st, bool soi) {
-  scatter_kmatrix_kernel<NZ, R><<<grid, SCATTER_THREADS, 0, st>>>(a);
-  if constexpr (std::is_same<R, double>::value)
-    if (soi) scatter_soi_k_kernel<NZ><<<grid, SCATTER_THREADS, 0, st>>>(a);
+template <int NZ>
+void launch_adding_front(const ScatterArgs<float>& a, dim3 grid, cudaStream_t st) {
+  adding_front_kernel<NZ><<<grid, SCATTER_THREADS, 0, st>>>(a);
 }
 
 template <int NZ, class R, class C>
@@ -30,7 +28,7 @@ void launch_scatter_reverse(const ScatterArgs<R>& a, unsigned grid, cudaStream_t
 }
 
 template void launch_scatter_layers_k<5, float, float>(const ScatterArgs<float>&, unsigned, cudaStream_t);
-template void launch_scatter_kmatrix<5, float>(const ScatterArgs<float>&, dim3, cudaStream_t, bool);
+template void launch_adding_front<5>(const ScatterArgs<float>&, dim3, cudaStream_t);
 template void launch_scatter_reverse<5, float, float>(const ScatterArgs<float>&, unsigned, cudaStream_t);
 
 }  // namespace crtm

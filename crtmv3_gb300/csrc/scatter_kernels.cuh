@@ -478,6 +478,30 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_kmatrix_kernel(Scatte
   cb[3 * (size_t)L] = a.cover[p] >= 0.0 ? clear_column_radiance(c, a.TAU + (size_t)p * Kmax * L + l, L) : 0.0;
 }
 
+// Before adding_team_kernel, one thread per (profile, channel): the radiance
+// of the clear column of a fractional profile (FP64), and the failure of a
+// stream set that does not fit.
+template <int NZ>
+__global__ void __launch_bounds__(SCATTER_THREADS) adding_front_kernel(ScatterArgs<float> a) {
+  constexpr int NE = layer_record<NZ>();
+  const int L = a.L, Kmax = a.Kmax;
+  const int p = blockIdx.y, gp = batch_profile(a.b, a.p_begin + p);
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= L || a.pv.status[p] != 0) return;
+  const CloudyColumn c = column_inputs(a, p, gp, l);
+  if (c.n_clouds == 0 && c.n_aerosols == 0) return;
+  double* cb = a.CB + (size_t)p * 4 * L + l;
+  cb[3 * (size_t)L] = a.cover[p] >= 0.0 ? clear_column_radiance(c, a.TAU + (size_t)p * Kmax * L + l, L) : 0.0;
+  StreamSet<NZ, double> S;
+  const int code = stream_set<NZ, double>(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, c_gauss, S);
+  if (!code) return;
+  if (a.x.nfs) a.x.nfs[(size_t)gp * L + a.sp.out[l]] = c.nleg + 2;
+  atomicCAS(a.error, 0, code);
+  if (a.status) atomicOr(a.status + gp, 1 << 4);
+  cb[0] = cb[(size_t)L] = cb[2 * (size_t)L] = 0.0;
+  for (int k = 0; k < c.Ku; k++) a.LBA[((size_t)p * Kmax + k) * NE * L + l] = -1.0f;
+}
+
 // K-matrix / adjoint of the SOI profiles (Options%RT_Algorithm_Id = RT_SOI),
 // one thread per (profile, channel): the orders of interaction over the FP64
 // layer records with every order's fields kept in FS (checkpoints and

@@ -1,6 +1,6 @@
 // Host launchers of the scattering K-matrix/adjoint kernels.  R is the gas
 // optics' arithmetic (double in the FP64 form, float in the mixed form), C
-// the layer solver's (the same); the adding and its adjoint are FP64 in both.
+// the layer solver's (the same); the adding and its adjoint are in R too.
 // A batch with SOI profiles runs in the FP64 form.  Translation units per
 // angle capacity (d5: the stream rule's 2-6 streams, d10: Options%n_Streams
 // up to 16): scatter_k_*.cu (records, adding adjoint, reverse sweep of the ADA
@@ -22,17 +22,25 @@ int scatter_k_d5f_set_gauss(const GaussTable& g);
 int scatter_k_d10f_set_gauss(const GaussTable& g);
 int scatter_soi_d5_set_gauss(const GaussTable& g);
 int scatter_soi_d10_set_gauss(const GaussTable& g);
+int scatter_team_set_gauss(const GaussTable& g);
 inline int scatter_k_set_gauss(const GaussTable& g) {
   return scatter_k_d5_set_gauss(g) | scatter_k_d10_set_gauss(g) | scatter_k_d5f_set_gauss(g) |
-         scatter_k_d10f_set_gauss(g) | scatter_soi_d5_set_gauss(g) | scatter_soi_d10_set_gauss(g);
+         scatter_k_d10f_set_gauss(g) | scatter_soi_d5_set_gauss(g) | scatter_soi_d10_set_gauss(g) |
+         scatter_team_set_gauss(g);
 }
 
 // layer records (in R) with the layer solver in C
 template <int NZ, class R, class C>
 void launch_scatter_layers_k(const ScatterArgs<R>& a, unsigned grid, cudaStream_t st);
-// the ADA adding adjoint, then (FP64 form, soi) the SOI orders' adjoint of the SOI profiles
+// FP64 form: the ADA adding adjoint, then (soi) the SOI orders' adjoint of the SOI profiles
 template <int NZ, class R>
 void launch_scatter_kmatrix(const ScatterArgs<R>& a, dim3 grid, cudaStream_t st, bool soi);
+// mixed form: the clear columns and refused stream sets, then the ADA adding
+// and its adjoint by teams of lanes (NC: angle capacity of the records; returns
+// the number of kernels launched)
+template <int NZ>
+void launch_adding_front(const ScatterArgs<float>& a, dim3 grid, cudaStream_t st);
+int launch_adding_team(const ScatterArgs<float>& a, int NC, cudaStream_t st);
 // the ADA profiles' layer contraction (reverse sweep in C)
 template <int NZ, class R, class C>
 void launch_scatter_reverse(const ScatterArgs<R>& a, unsigned grid, cudaStream_t st);
