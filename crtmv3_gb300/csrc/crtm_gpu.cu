@@ -841,7 +841,8 @@ struct Work {
   double* ras;      // adjoint: [n][nv][K]
   double* pts;      // adjoint: [n][Kmax]
   double* tss;      // adjoint: [n]
-  int* idx_map;     // [Jm]
+  unsigned* LIST;   // mixed form, scattering: [classes + 1][n][Kmax][L] item lists
+  int* idx_map;     // [Jm], then (from MAX_ABS) the lists' counters
 };
 
 template <int G, class R> struct Tune;
@@ -906,6 +907,8 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
       wk.LBK = (R*)carve(nn * Kmax * (size_t)sw.rec * L * sizeof(R));
     else
       wk.LB = (R*)carve(nn * Kmax * (size_t)sw.rec * L * sizeof(R));
+    if (sizeof(R) == sizeof(float) && !sw.soi)
+      wk.LIST = (unsigned*)carve(nn * Kmax * L * ((sw.nz <= 5 ? 5 : SC_NZ_MAX) + 1) * sizeof(unsigned));
     wk.maxreff = (double*)carve(nn * sizeof(double));
     wk.cover = (double*)carve(nn * sizeof(double));
     // SOI fields: 2 fields x 2 buffers x levels x angles
@@ -939,7 +942,7 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
     wk.pts = (double*)carve(nn * Kmax * sizeof(double));
     wk.tss = (double*)carve(nn * sizeof(double));
   }
-  wk.idx_map = (int*)carve(MAX_ABS * sizeof(int));
+  wk.idx_map = (int*)carve((MAX_ABS + SC_NZ_MAX + 2) * sizeof(int));
   if (w) *w = wk;
   return off;
 }
@@ -1180,6 +1183,8 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
   const size_t per = work_bytes<G, R>(s, 64, Kmax, nv, mode, nullptr, nullptr, sw) / 64 + 1;
   int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)P, h->workspace_budget / per));
   if (hc && hc->max_chunk > 0) chunk = std::min(chunk, hc->max_chunk);
+  if (scat && sizeof(R) == sizeof(float))   // the scattering item lists hold 32-bit counts and indices
+    chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)chunk, (size_t)0x7fffffff / ((size_t)Kmax * L)));
   constexpr int form = sizeof(R) == sizeof(float) ? 1 : 0;
   if (!fixed && s.tune_chunk[form] > 0) chunk = std::min(chunk, s.tune_chunk[form]);
   char* ws_base;
@@ -1294,32 +1299,49 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
       const long long nlay = (long long)n * Kmax * L;
       const unsigned gl = (unsigned)((nlay + SCATTER_THREADS - 1) / SCATTER_THREADS);
       dim3 ga((L + SCATTER_THREADS - 1) / SCATTER_THREADS, n);
+      constexpr bool mixed = std::is_same<R, float>::value;
+      const bool listed = mixed && !soi;
+      const ItemLists lists{w.idx_map + MAX_ABS, w.LIST, (size_t)nlay, nz_max ? SC_NZ_MAX : 5};
       {
         StageScope sc(h, 6, st);
         scatter_profile_kernel<R><<<(n + 3) / 4, 128, 0, st>>>(sa);
         CK_LAUNCH(h);
-        if (split) {   // K-matrix / adjoint: FP64 records, layer solver in R
-          if (nz_max)
-            launch_scatter_layers_k<SC_NZ_MAX, R, R>(sa, gl, st);
-          else
-            launch_scatter_layers_k<5, R, R>(sa, gl, st);
-        } else if (soi) {   // forward with SOI profiles: FP64 layer solver (records in R)
+        if (listed) {   // mixed form: layers by lists
+          if constexpr (mixed) {
+            if (cudaMemsetAsync(lists.count, 0, (lists.n_class + 2) * sizeof(int), st) != cudaSuccess)
+              return fail(h, "cudaMemsetAsync failed");
+            scatter_classify_kernel<<<(unsigned)((nlay + CLASSIFY_THREADS - 1) / CLASSIFY_THREADS), CLASSIFY_THREADS, 0,
+                                      st>>>(sa, lists.n_class, lists);
+            CK_LAUNCH(h);
+            float* rec = split ? w.LBK : w.LB;
+            for (int pass = 0; pass <= 1; pass++) {
+              if (nz_max)
+                launch_layers_listed<SC_NZ_MAX>(sa, rec, lists, pass, st);
+              else
+                launch_layers_listed<5>(sa, rec, lists, pass, st);
+              CK_LAUNCH(h);
+            }
+          }
+        } else if (split) {   // FP64 K-matrix / adjoint
+          if constexpr (!mixed) {
+            if (nz_max)
+              launch_scatter_layers_k<SC_NZ_MAX, R, R>(sa, gl, st);
+            else
+              launch_scatter_layers_k<5, R, R>(sa, gl, st);
+            CK_LAUNCH(h);
+          }
+        } else {   // forward: FP64 form, or SOI profiles (FP64 layer solver, records in R)
           if (nz_max)
             scatter_layers_kernel<SC_NZ_MAX, R, R, double><<<gl, SCATTER_THREADS, 0, st>>>(sa, w.LB);
           else
             scatter_layers_kernel<5, R, R, double><<<gl, SCATTER_THREADS, 0, st>>>(sa, w.LB);
-        } else {   // forward: layer solver in R (records in R)
-          if (nz_max)
-            scatter_layers_kernel<SC_NZ_MAX, R, R, R><<<gl, SCATTER_THREADS, 0, st>>>(sa, w.LB);
-          else
-            scatter_layers_kernel<5, R, R, R><<<gl, SCATTER_THREADS, 0, st>>>(sa, w.LB);
+          CK_LAUNCH(h);
         }
-        CK_LAUNCH(h);
       }
       if (split) {
         {
           StageScope sc(h, 7, st);
-          if constexpr (std::is_same<R, float>::value) {
+          if constexpr (mixed) {
             if (soi) return fail(h, "internal: SOI K-matrix in the mixed form");
             if (nz_max)
               launch_adding_front<SC_NZ_MAX>(sa, ga, st);
@@ -1336,11 +1358,21 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
         }
         {
           StageScope sc(h, 8, st);
-          if (nz_max)
-            launch_scatter_reverse<SC_NZ_MAX, R, R>(sa, gl, st);
-          else
-            launch_scatter_reverse<5, R, R>(sa, gl, st);
-          CK_LAUNCH(h);
+          if constexpr (mixed) {
+            for (int pass = 0; pass <= 2; pass += 2) {
+              if (nz_max)
+                launch_reverse_listed<SC_NZ_MAX>(sa, lists, pass, st);
+              else
+                launch_reverse_listed<5>(sa, lists, pass, st);
+              CK_LAUNCH(h);
+            }
+          } else {
+            if (nz_max)
+              launch_scatter_reverse<SC_NZ_MAX, R, R>(sa, gl, st);
+            else
+              launch_scatter_reverse<5, R, R>(sa, gl, st);
+            CK_LAUNCH(h);
+          }
           if constexpr (std::is_same<R, double>::value) {
             if (soi) {   // the SOI profiles' layers
               if (nz_max)

@@ -597,12 +597,13 @@ CRTM_HD int bulk_to_inputs(const CloudyColumn& in, const CloudLut& lut, int nleg
 // scattering, 0 clear) or a negative error; kind_rec is the record's kind
 // (the forward's); a mismatch returns -7.  In FP32, *in_fp64 is set (and
 // nothing written) where the layer must be taken in FP64; layer_adjoint
-// below then runs the FP64 instance.
+// below then runs the FP64 instance.  defer: a layer that needs shifted sensor
+// angles or FP64 is not taken; returns LAYER_DEFERRED.
 template <int NZ, class T>
 CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const StreamSet<NZ, double>& St, int k,
                              double gas_od, int kind_rec, const Mat<NZ, double>& T_b, const Mat<NZ, double>& R_b,
                              const double* src_b, double od_b, double B_b, double* g, double (*gs)[3],
-                             bool* in_fp64) {
+                             bool* in_fp64, bool defer) {
   constexpr bool fp32 = std::is_same<T, float>::value;
   const int nleg = St.nleg, nS = St.nS, nZ = St.nZ;
   // the layer's bulk optics in FP64 (the combine's adjoint needs them there;
@@ -664,6 +665,7 @@ CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const 
     bool rich = false;
     const double gap_min = fp32 ? FP32_ADJ_GAP_MIN : SENSOR_GAP_MIN;
     if (gap < gap_min && nZ == nS + 1) {
+      if (defer) return LAYER_DEFERRED;
       // A quadrature eigenvalue of MOM nearly meets the sensor angle's: the
       // derivatives through the nearly defective eigenbasis lose about
       // eps / gap^2.  T, R and the source are smooth in the sensor angle, so
@@ -731,15 +733,17 @@ CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const 
 template <int NZ, class T>
 CRTM_HD int layer_adjoint(const CloudyColumn& in, const CloudLut& lut, const StreamSet<NZ, double>& St, int k,
                           double gas_od, int kind_rec, const Mat<NZ, double>& T_b, const Mat<NZ, double>& R_b,
-                          const double* src_b, double od_b, double B_b, double* g, double (*gs)[3]) {
+                          const double* src_b, double od_b, double B_b, double* g, double (*gs)[3], bool defer) {
   bool in_fp64 = false;
   const int r = layer_adjoint_in<NZ, T>(in, lut, St, k, gas_od, kind_rec, T_b, R_b, src_b, od_b, B_b, g, gs,
-                                        &in_fp64);
+                                        &in_fp64, defer);
   if constexpr (std::is_same<T, float>::value) {
     // one call site of the FP64 instance for every FP32 fallback
-    if (in_fp64)
+    if (in_fp64) {
+      if (defer) return LAYER_DEFERRED;
       return layer_adjoint_in<NZ, double>(in, lut, St, k, gas_od, kind_rec, T_b, R_b, src_b, od_b, B_b, g, gs,
-                                          &in_fp64);
+                                          &in_fp64, false);
+    }
   }
   return r;
 }

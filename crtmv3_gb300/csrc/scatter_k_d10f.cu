@@ -1,8 +1,6 @@
-// Scattering K-matrix/adjoint kernels for NZ = 10 angles (Options%n_Streams up to 16), mixed form (FP32 gas optics and layer solver, FP64 adding):
-// the layer records, the adding adjoint (and, FP64 form, the SOI orders'
-// adjoint), and the reverse sweep through the ADA layers' optics.  One
-// translation unit per angle capacity and form so that the library compiles
-// in parallel.
+// The mixed form's per-thread scattering kernels for NZ = 10 angles (Options%n_Streams up to 16):
+// the layer records, what precedes the adding, and the reverse sweep through
+// the layers' optics.
 #include "scatter_kernels.cuh"
 #include "scatter_launch.h"
 
@@ -12,9 +10,9 @@ int scatter_k_d10f_set_gauss(const GaussTable& g) {
   return cudaMemcpyToSymbol(c_gauss, &g, sizeof g) == cudaSuccess ? 0 : 1;
 }
 
-template <int NZ, class R, class C>
-void launch_scatter_layers_k(const ScatterArgs<R>& a, unsigned grid, cudaStream_t st) {
-  scatter_layers_kernel<NZ, R, R, C><<<grid, SCATTER_THREADS, 0, st>>>(a, a.LBK);
+template <int NZ>
+void launch_layers_listed(const ScatterArgs<float>& a, float* rec, const ItemLists& ls, int pass, cudaStream_t st) {
+  layers_listed_kernel<NZ><<<list_ctas(ls, pass), list_threads(pass), 0, st>>>(a, rec, ls, pass);
 }
 
 template <int NZ>
@@ -22,13 +20,13 @@ void launch_adding_front(const ScatterArgs<float>& a, dim3 grid, cudaStream_t st
   adding_front_kernel<NZ><<<grid, SCATTER_THREADS, 0, st>>>(a);
 }
 
-template <int NZ, class R, class C>
-void launch_scatter_reverse(const ScatterArgs<R>& a, unsigned grid, cudaStream_t st) {
-  scatter_reverse_kernel<NZ, R, C><<<grid, SCATTER_THREADS, 0, st>>>(a);
+template <int NZ>
+void launch_reverse_listed(const ScatterArgs<float>& a, const ItemLists& ls, int pass, cudaStream_t st) {
+  reverse_listed_kernel<NZ><<<list_ctas(ls, pass), list_threads(pass), 0, st>>>(a, ls, pass);
 }
 
-template void launch_scatter_layers_k<10, float, float>(const ScatterArgs<float>&, unsigned, cudaStream_t);
+template void launch_layers_listed<10>(const ScatterArgs<float>&, float*, const ItemLists&, int, cudaStream_t);
 template void launch_adding_front<10>(const ScatterArgs<float>&, dim3, cudaStream_t);
-template void launch_scatter_reverse<10, float, float>(const ScatterArgs<float>&, unsigned, cudaStream_t);
+template void launch_reverse_listed<10>(const ScatterArgs<float>&, const ItemLists&, int, cudaStream_t);
 
 }  // namespace crtm

@@ -223,31 +223,47 @@ __device__ __forceinline__ CloudyColumn column_inputs(const ScatterArgs<R>& a, i
   return c;
 }
 
+// Active species of layer k (clouds above the water-content threshold after
+// the cover scaling and not dropped, aerosols above theirs for non-microwave
+// sensors), as seed indices of layer_optics.
+CRTM_HD int active_species(const CloudyColumn& c, int k, int* sp) {
+  int n = 0;
+  if (!(c.cf && c.cf[k] < MIN_COVERAGE))
+    for (int i = 0; i < c.n_clouds; i++)
+      if (c.wc[i * c.cstride + k] / c.wc_div > WATER_CONTENT_THRESHOLD) sp[n++] = i;
+  if (!c.microwave)
+    for (int i = 0; i < c.n_aerosols; i++)
+      if (c.conc[i * c.cstride + k] > AEROSOL_CONTENT_THRESHOLD) sp[n++] = c.n_clouds + i;
+  return n;
+}
+
+// One layer's record by one thread, item idx of the chunk (channels fastest).
+// defer: returns true, with nothing written, for a layer that layer_optics defers.
 template <int NZ, class R, class Rec, class C>
-__global__ void __launch_bounds__(SCATTER_THREADS) scatter_layers_kernel(ScatterArgs<R> a, Rec* LBr) {
+__device__ __forceinline__ bool scatter_layer_item(const ScatterArgs<R>& a, Rec* LBr, long long idx, bool defer) {
   constexpr int NE = layer_record<NZ>();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int L = a.L, Kmax = a.Kmax;
-  if (idx >= (long long)a.n_chunk * Kmax * L) return;
+  if (idx >= (long long)a.n_chunk * Kmax * L) return false;
   const int l = (int)(idx % L);
   const int k = (int)((idx / L) % Kmax);
   const int p = (int)(idx / ((long long)L * Kmax));
   const int gp = batch_profile(a.b, a.p_begin + p);
-  if (a.pv.status[p] != 0 || k >= a.b.n_layers[gp]) return;
+  if (a.pv.status[p] != 0 || k >= a.b.n_layers[gp]) return false;
   Rec* rec = LBr + ((size_t)p * Kmax + k) * NE * L + l;
   const CloudyColumn c = column_inputs(a, p, gp, l);
-  if (c.n_clouds == 0 && c.n_aerosols == 0) return;
+  if (c.n_clouds == 0 && c.n_aerosols == 0) return false;
   StreamSet<NZ, double> S;
   if (int rc = stream_set<NZ, double>(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, c_gauss, S)) {
     rec[0] = Rec(-rc);
-    return;
+    return false;
   }
   Mat<NZ, Rec> Tm, Rm;
   Rec src[NZ], od;
   const double gas = double(a.TAU[((size_t)p * Kmax + k) * L + l]);
   double bs = 0.0;
   const int kind = layer_optics<NZ, Rec, C>(c, a.lut, S, k, C(gas), C(c.temperature[k]), &od, Tm, Rm, src,
-                                            NoSeed(), nullptr, a.x.sod ? &bs : nullptr);
+                                            NoSeed(), nullptr, a.x.sod ? &bs : nullptr, defer);
+  if (kind == LAYER_DEFERRED) return true;
   if (kind >= 0) {
     const size_t pl = (size_t)gp * L + a.sp.out[l];
     if (a.x.lod) a.x.lod[pl * Kmax + k] = double(od);
@@ -255,7 +271,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_layers_kernel(Scatter
   }
   rec[0] = Rec(kind);
   rec[(size_t)L] = od;
-  if (kind != 1) return;
+  if (kind != 1) return false;
   const int nZ = S.nZ;
   for (int i = 0; i < nZ; i++)
     for (int j = 0; j < nZ; j++) {
@@ -263,6 +279,128 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_layers_kernel(Scatter
       rec[(size_t)(2 + NZ * NZ + i * NZ + j) * L] = Rm.a[i][j];
     }
   for (int i = 0; i < nZ; i++) rec[(size_t)(2 + 2 * NZ * NZ + i) * L] = src[i];
+  return false;
+}
+
+template <int NZ, class R, class Rec, class C>
+__global__ void __launch_bounds__(SCATTER_THREADS) scatter_layers_kernel(ScatterArgs<R> a, Rec* LBr) {
+  scatter_layer_item<NZ, R, Rec, C>(a, LBr, (long long)blockIdx.x * blockDim.x + threadIdx.x, false);
+}
+
+// ---- mixed form: the layers by lists.  Lanes of a warp that take channels in
+// order meet clear layers, angle counts from 2 to 10 and, in a few percent of
+// the layers, shifted sensor angles or FP64, which cost 5 to 60 times a plain
+// layer and which the whole warp waits for: of 32 lanes 12 were active, and
+// the warps of an SM, each elsewhere in the code, waited for instructions.
+// Here a warp's layers are of one class (ItemLists), and what FP32 cannot take
+// in one solve is left for a second pass.  2000 profiles x 16 microwave
+// channels, adjoint: layers 57.9 -> 24.0 ms, reverse sweep 138 -> 80.5 ms.
+struct ItemLists {
+  int* count;        // [n_class + 2]: the classes', then two lists of deferred items
+  unsigned* items;   // [n_class + 1][cap] indices in the chunk
+  size_t cap;
+  int n_class;       // class 0: nothing scatters; else the number of angles - 1
+};
+
+// Angles of a (profile, channel): stream_set's counts and error codes.
+struct StreamShape { int nS, nZ, isat; };
+__device__ __forceinline__ int stream_shape(int nleg, double mu_sensor, int lut_nleg, int NC, StreamShape& s) {
+  const int loff = legendre_offset(nleg);
+  if (loff < 0 || nleg > SC_NLEG_MAX) return 1;
+  if (lut_nleg >= 0 && lut_nleg < nleg + loff) return 2;   // lut_nleg < 0: no clouds
+  s.nS = (nleg + 2) / 2;
+  if (s.nS + 1 > NC || s.nS > 9) return 3;
+  s.nZ = s.nS;
+  s.isat = -1;
+  for (int i = 0; i < s.nS; i++)
+    if (s.isat < 0 && fabs(c_gauss.mu[s.nS][i] - mu_sensor) < ANGLE_THRESHOLD) s.isat = i;
+  if (s.isat < 0) { s.nZ = s.nS + 1; s.isat = s.nS; }
+  return 0;
+}
+
+constexpr int CLASSIFY_THREADS = 256;
+// The class of every item of the chunk that has something to do, onto the
+// lists (a class only groups items; any is right).
+static __global__ void __launch_bounds__(CLASSIFY_THREADS) scatter_classify_kernel(ScatterArgs<float> a, int NC,
+                                                                                   ItemLists ls) {
+  constexpr int W = CLASSIFY_THREADS / 32;
+  __shared__ int cnt[W][SC_NZ_MAX], base[SC_NZ_MAX];
+  const long long idx = (long long)blockIdx.x * CLASSIFY_THREADS + threadIdx.x;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, L = a.L, Kmax = a.Kmax;
+  int cls = -1;
+  if (idx < (long long)a.n_chunk * Kmax * L) {
+    const int l = (int)(idx % L), k = (int)((idx / L) % Kmax), p = (int)(idx / ((long long)L * Kmax));
+    const int gp = batch_profile(a.b, a.p_begin + p);
+    if (a.pv.status[p] == 0 && k < a.b.n_layers[gp]) {
+      const CloudyColumn c = column_inputs(a, p, gp, l);
+      if (c.n_clouds > 0 || c.n_aerosols > 0) {
+        StreamShape s{0, 1, 0};
+        int sp[2 * SC_NC_MAX];
+        const bool bad = stream_shape(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, NC, s);
+        cls = bad || active_species(c, k, sp) == 0 ? 0 : s.nZ - 1;
+      }
+    }
+  }
+  int rank = 0;
+  for (int q = 0; q < ls.n_class; q++) {
+    const unsigned m = __ballot_sync(FULL, cls == q);
+    if (cls == q) rank = __popc(m & ((1u << lane) - 1u));
+    if (lane == 0) cnt[wib][q] = __popc(m);
+  }
+  __syncthreads();
+  if (threadIdx.x < ls.n_class) {
+    int n = 0;
+    for (int w = 0; w < W; w++) {
+      const int v = cnt[w][threadIdx.x];
+      cnt[w][threadIdx.x] = n;
+      n += v;
+    }
+    base[threadIdx.x] = n ? atomicAdd(ls.count + threadIdx.x, n) : 0;
+  }
+  __syncthreads();
+  if (cls >= 0) ls.items[(size_t)cls * ls.cap + base[cls] + cnt[wib][cls] + rank] = (unsigned)idx;
+}
+
+// A thread's item of a pass: 0 the classes one after another from the most
+// angles down, each from a CTA's first thread on; 1, 2 the items deferred by
+// the layers' and by the reverse sweep's first pass.
+__device__ __forceinline__ bool listed_item(const ItemLists& ls, int pass, long long& idx) {
+  if (pass > 0) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ls.count[ls.n_class + pass - 1]) return false;
+    idx = ls.items[(size_t)ls.n_class * ls.cap + i];
+    return true;
+  }
+  int c0 = blockIdx.x;
+  for (int q = ls.n_class - 1; q >= 0; q--) {
+    const int n = ls.count[q], nb = (n + SCATTER_THREADS - 1) / SCATTER_THREADS;
+    if (c0 < nb) {
+      const int i = c0 * SCATTER_THREADS + threadIdx.x;
+      if (i >= n) return false;
+      idx = ls.items[(size_t)q * ls.cap + i];
+      return true;
+    }
+    c0 -= nb;
+  }
+  return false;
+}
+__device__ __forceinline__ void defer_item(const ItemLists& ls, int pass, long long idx) {
+  ls.items[(size_t)ls.n_class * ls.cap + atomicAdd(ls.count + ls.n_class + pass - 1, 1)] = (unsigned)idx;
+}
+// Threads and CTAs of a pass, for all of a chunk's items however they divide
+// (the counts are on the device; CTAs beyond them end at once).  Deferred
+// items are few and long: one warp a CTA, spread over the SMs.
+inline unsigned list_threads(int pass) { return pass ? 32 : SCATTER_THREADS; }
+inline unsigned list_ctas(const ItemLists& ls, int pass) {
+  return (unsigned)((ls.cap + list_threads(pass) - 1) / list_threads(pass) + (pass ? 0 : ls.n_class));
+}
+
+template <int NZ>
+__global__ void __launch_bounds__(SCATTER_THREADS) layers_listed_kernel(ScatterArgs<float> a, float* LBr, ItemLists ls,
+                                                                        int pass) {
+  long long idx;
+  if (!listed_item(ls, pass, idx)) return;
+  if (scatter_layer_item<NZ, float, float, float>(a, LBr, idx, pass == 0)) defer_item(ls, 1, idx);
 }
 
 // The forward's further RTSolution components of pair pl (profile p of the
@@ -569,20 +707,6 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_soi_k_kernel(ScatterA
   cb[3 * (size_t)L] = a.cover[p] >= 0.0 ? clear_column_radiance(c, a.TAU + (size_t)p * Kmax * L + l, L) : 0.0;
 }
 
-// Active species of layer k (clouds above the water-content threshold after
-// the cover scaling and not dropped, aerosols above theirs for non-microwave
-// sensors), as seed indices of layer_optics.
-CRTM_HD int active_species(const CloudyColumn& c, int k, int* sp) {
-  int n = 0;
-  if (!(c.cf && c.cf[k] < MIN_COVERAGE))
-    for (int i = 0; i < c.n_clouds; i++)
-      if (c.wc[i * c.cstride + k] / c.wc_div > WATER_CONTENT_THRESHOLD) sp[n++] = i;
-  if (!c.microwave)
-    for (int i = 0; i < c.n_aerosols; i++)
-      if (c.conc[i * c.cstride + k] > AEROSOL_CONTENT_THRESHOLD) sp[n++] = c.n_clouds + i;
-  return n;
-}
-
 template <int NZ, class R, class C>
 __global__ void __launch_bounds__(SCATTER_THREADS) scatter_contract_kernel(ScatterArgs<R> a) {
   constexpr int NE = layer_record<NZ>();
@@ -674,23 +798,21 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_contract_kernel(Scatt
 // profile not on SOI), one thread per (profile, layer, channel), by the
 // reverse sweep through the layer's optics (layer_adjoint): all of the
 // layer's inputs in one pass, in the arithmetic C.
-// (FP32 sweep with 10 angles: 3 CTAs per SM, 168 registers, measured 8 %
-// faster than the register-limited 2; the 5-angle sweep is fastest at 2)
+// defer: returns true, with nothing of it written, for a layer that
+// layer_adjoint defers.
 template <int NZ, class R, class C>
-__global__ void __launch_bounds__(SCATTER_THREADS, (NZ > 5 && sizeof(C) == 4) ? 3 : 1)
-    scatter_reverse_kernel(ScatterArgs<R> a) {
+__device__ __forceinline__ bool scatter_reverse_item(const ScatterArgs<R>& a, long long idx, bool defer) {
   constexpr int NE = layer_record<NZ>();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int L = a.L, Kmax = a.Kmax;
-  if (idx >= (long long)a.n_chunk * Kmax * L) return;
+  if (idx >= (long long)a.n_chunk * Kmax * L) return false;
   const int l = (int)(idx % L);
   const int k = (int)((idx / L) % Kmax);
   const int p = (int)(idx / ((long long)L * Kmax));
   const int gp = batch_profile(a.b, a.p_begin + p);
-  if (a.pv.status[p] != 0 || k >= a.b.n_layers[gp]) return;
+  if (a.pv.status[p] != 0 || k >= a.b.n_layers[gp]) return false;
   const CloudyColumn c = column_inputs(a, p, gp, l);
-  if (c.n_clouds == 0 && c.n_aerosols == 0) return;
-  if (c.soi) return;    // SOI profiles: scatter_contract_kernel
+  if (c.n_clouds == 0 && c.n_aerosols == 0) return false;
+  if (c.soi) return false;    // SOI profiles: scatter_contract_kernel
   const size_t kl = ((size_t)p * Kmax + k) * L + l;
   auto slot = [&](int s) { return s < c.n_clouds ? s : a.max_clouds + (s - c.n_clouds); };
   auto jac = [&](double* X, int s) -> double& {
@@ -707,10 +829,10 @@ __global__ void __launch_bounds__(SCATTER_THREADS, (NZ > 5 && sizeof(C) == 4) ? 
   if (kind < 0) {
     a.TODc[kl] = R(0);
     a.PT[kl] = R(0);
-    return;
+    return false;
   }
   StreamSet<NZ, double> S;
-  if (stream_set<NZ, double>(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, c_gauss, S)) return;
+  if (stream_set<NZ, double>(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, c_gauss, S)) return false;
   const int nZ = S.nZ;
   Mat<NZ, double> T_b, R_b;
   double src_b[NZ];
@@ -725,13 +847,14 @@ __global__ void __launch_bounds__(SCATTER_THREADS, (NZ > 5 && sizeof(C) == 4) ? 
     }
   double g[2], gs[2 * SC_NC_MAX][3];
   const int kr = layer_adjoint<NZ, C>(c, a.lut, S, k, double(a.TAU[kl]), kind, T_b, R_b, src_b,
-                                      kind == 1 ? 0.0 : od_b, B_b, g, gs);
+                                      kind == 1 ? 0.0 : od_b, B_b, g, gs, defer);
+  if (kr == LAYER_DEFERRED) return true;
   if (kr < 0) {
     atomicCAS(a.error, 0, -kr);
     if (a.status) atomicOr(a.status + gp, 1 << 4);
     a.TODc[kl] = R(0);
     a.PT[kl] = R(0);
-    return;
+    return false;
   }
   a.TODc[kl] = R(g[0]);
   a.PT[kl] = R(g[1]);
@@ -743,6 +866,22 @@ __global__ void __launch_bounds__(SCATTER_THREADS, (NZ > 5 && sizeof(C) == 4) ? 
       if (a.CV && a.alut.scheme == AEROSOL_CMAQ && s >= c.n_clouds) jac(a.CV, slot(s)) = gs[s][2];
     }
   }
+  return false;
+}
+
+template <int NZ, class R, class C>
+__global__ void __launch_bounds__(SCATTER_THREADS) scatter_reverse_kernel(ScatterArgs<R> a) {
+  scatter_reverse_item<NZ, R, C>(a, (long long)blockIdx.x * blockDim.x + threadIdx.x, false);
+}
+// Mixed form: by the lists of the layers.  (10 angles: 3 CTAs per SM, 168
+// registers, measured 8 % faster than the register-limited 2; 5 angles are
+// fastest at 2.)
+template <int NZ>
+__global__ void __launch_bounds__(SCATTER_THREADS, NZ > 5 ? 3 : 1)
+    reverse_listed_kernel(ScatterArgs<float> a, ItemLists ls, int pass) {
+  long long idx;
+  if (!listed_item(ls, pass, idx)) return;
+  if (scatter_reverse_item<NZ, float, float>(a, idx, pass == 0)) defer_item(ls, 2, idx);
 }
 
 // Species and cloud-fraction Jacobians of one (profile, channel), in place:

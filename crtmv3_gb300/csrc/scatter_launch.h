@@ -14,6 +14,7 @@ namespace crtm {
 
 struct GaussTable;
 template <class R> struct ScatterArgs;
+struct ItemLists;
 
 // Upload the Gauss table into each unit's constant memory; 0 on success.
 int scatter_k_d5_set_gauss(const GaussTable& g);
@@ -29,7 +30,7 @@ inline int scatter_k_set_gauss(const GaussTable& g) {
          scatter_team_set_gauss(g);
 }
 
-// layer records (in R) with the layer solver in C
+// FP64 form: layer records (in R) with the layer solver in C
 template <int NZ, class R, class C>
 void launch_scatter_layers_k(const ScatterArgs<R>& a, unsigned grid, cudaStream_t st);
 // FP64 form: the ADA adding adjoint, then (soi) the SOI orders' adjoint of the SOI profiles
@@ -41,7 +42,13 @@ void launch_scatter_kmatrix(const ScatterArgs<R>& a, dim3 grid, cudaStream_t st,
 template <int NZ>
 void launch_adding_front(const ScatterArgs<float>& a, dim3 grid, cudaStream_t st);
 int launch_adding_team(const ScatterArgs<float>& a, int NC, cudaStream_t st);
-// the ADA profiles' layer contraction (reverse sweep in C)
+// mixed form: the listed layers' records and their reverse sweep; pass 0 the
+// classes' lists, then 1 (layers) or 2 (reverse) what it deferred
+template <int NZ>
+void launch_layers_listed(const ScatterArgs<float>& a, float* rec, const ItemLists& ls, int pass, cudaStream_t st);
+template <int NZ>
+void launch_reverse_listed(const ScatterArgs<float>& a, const ItemLists& ls, int pass, cudaStream_t st);
+// FP64 form: the ADA profiles' layer contraction (reverse sweep in C)
 template <int NZ, class R, class C>
 void launch_scatter_reverse(const ScatterArgs<R>& a, unsigned grid, cudaStream_t st);
 // the SOI profiles' layer contraction (derivative numbers, FP64 form)

@@ -1090,10 +1090,14 @@ CRTM_HD int species_sums(const CloudyColumn& in, const CloudLut& lut, int nleg, 
 // negative on failure.  bs_out (optional): the layer's scattering
 // coefficient before the delta truncation where it is significant, else 0
 // (its term of the scattering optical depth, CRTM_AtmOptics.f90:425-427).
+// defer: an FP32 layer that needs shifted sensor angles or FP64 is not solved;
+// returns LAYER_DEFERRED.  (A run-time choice: the code that solves the other
+// layers is then the same, and so are their bits.)
+constexpr int LAYER_DEFERRED = 2;
 template <int NZ, class T, class S = double, class Seed = NoSeed>
 CRTM_HD int layer_optics(const CloudyColumn& in, const CloudLut& lut, const StreamSet<NZ, double>& St, int k,
                          S gas_od, S tk, T* od_out, Mat<NZ, T>& Tm, Mat<NZ, T>& Rm, T* src,
-                         Seed seed = Seed(), double* gap = nullptr, double* bs_out = nullptr) {
+                         Seed seed = Seed(), double* gap = nullptr, double* bs_out = nullptr, bool defer = false) {
   const int nleg = St.nleg;
   S od = gas_od, bs_sum = S(0.0);
   S pcs[SC_NLEG_MAX + 1];
@@ -1137,6 +1141,7 @@ CRTM_HD int layer_optics(const CloudyColumn& in, const CloudLut& lut, const Stre
                                           gap ? gap : &g32);
     if constexpr (std::is_same<S, float>::value) {
       bool in_fp64 = !ok;
+      if (defer && (in_fp64 || ((gap ? *gap : g32) < FP32_GAP_MIN && St.nZ == St.nS + 1))) return LAYER_DEFERRED;
       if (ok && (gap ? *gap : g32) < FP32_GAP_MIN && St.nZ == St.nS + 1) {
         // the sensor angle nearly meets a MOM eigenvalue: the layer at sensor
         // angles mu (1 +- h), mu (1 +- 2h), combined as (4 M(h) - M(2h)) / 3

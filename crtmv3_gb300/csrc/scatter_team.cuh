@@ -28,22 +28,6 @@ __device__ __forceinline__ bool in_class(int nZ) {
   return NZ == 4 ? nZ <= 4 : (NZ == 10 ? nZ > 6 : nZ == NZ);
 }
 
-// Angles of a (profile, channel): stream_set's counts and error codes.
-struct StreamShape { int nS, nZ, isat; };
-__device__ __forceinline__ int stream_shape(int nleg, double mu_sensor, int lut_nleg, int NC, StreamShape& s) {
-  const int loff = legendre_offset(nleg);
-  if (loff < 0 || nleg > SC_NLEG_MAX) return 1;
-  if (lut_nleg >= 0 && lut_nleg < nleg + loff) return 2;   // lut_nleg < 0: no clouds
-  s.nS = (nleg + 2) / 2;
-  if (s.nS + 1 > NC || s.nS > 9) return 3;
-  s.nZ = s.nS;
-  s.isat = -1;
-  for (int i = 0; i < s.nS; i++)
-    if (s.isat < 0 && fabs(c_gauss.mu[s.nS][i] - mu_sensor) < ANGLE_THRESHOLD) s.isat = i;
-  if (s.isat < 0) { s.nZ = s.nS + 1; s.isat = s.nS; }
-  return 0;
-}
-
 constexpr int ADD_MATS = 10, ADD_VECS = 4;
 template <int NZ>
 constexpr size_t adding_team_smem() {
