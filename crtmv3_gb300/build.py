@@ -13,9 +13,10 @@ LIB = os.path.join(HERE, "libcrtm_gb300.so")
 # scattering K-matrix kernels per arithmetic form and one of the SOI layers'
 # contraction.
 SOURCES = ["crtm_gpu.cu", "scatter_k_d5.cu", "scatter_k_d10.cu", "scatter_k_d5f.cu", "scatter_k_d10f.cu",
-           "scatter_soi_d5.cu", "scatter_soi_d10.cu", "scatter_team.cu"]
+           "scatter_soi_d5.cu", "scatter_soi_d10.cu", "scatter_team.cu", "scatter_k_d5x.cu"]
 HEADERS = ["odps_physics.cuh", "odps_prep.cuh", "odps_kernels.cuh", "optran.cuh", "scatter_physics.cuh",
-           "scatter_kernels.cuh", "scatter_team.cuh", "scatter_team_math.cuh", "scatter_adjoint.cuh", "scatter_launch.h", "dual.cuh", "dd.cuh"]
+           "scatter_kernels.cuh", "scatter_team.cuh", "scatter_team_math.cuh", "scatter_adjoint.cuh",
+           "scatter_fixed.cuh", "scatter_launch.h", "dual.cuh", "dd.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "--expt-relaxed-constexpr", "-lineinfo", "-Xcompiler", "-fPIC"]
 

@@ -1314,6 +1314,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
                                       st>>>(sa, lists.n_class, lists);
             CK_LAUNCH(h);
             float* rec = split ? w.LBK : w.LB;
+            if (!nz_max) h->launches += launch_layers_fixed(sa, rec, lists, st);
             for (int pass = 0; pass <= 1; pass++) {
               if (nz_max)
                 launch_layers_listed<SC_NZ_MAX>(sa, rec, lists, pass, st);
@@ -1359,6 +1360,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
         {
           StageScope sc(h, 8, st);
           if constexpr (mixed) {
+            if (!nz_max) h->launches += launch_reverse_fixed(sa, lists, st);
             for (int pass = 0; pass <= 2; pass += 2) {
               if (nz_max)
                 launch_reverse_listed<SC_NZ_MAX>(sa, lists, pass, st);

@@ -25,7 +25,7 @@
 //     which costs a few LUT evaluations and no matrix work.
 #pragma once
 
-#include "scatter_physics.cuh"
+#include "scatter_fixed.cuh"
 
 namespace crtm {
 
@@ -599,7 +599,8 @@ CRTM_HD int bulk_to_inputs(const CloudyColumn& in, const CloudLut& lut, int nleg
 // nothing written) where the layer must be taken in FP64; layer_adjoint
 // below then runs the FP64 instance.  defer: a layer that needs shifted sensor
 // angles or FP64 is not taken; returns LAYER_DEFERRED.
-template <int NZ, class T>
+// NS: as in layer_optics.
+template <int NZ, class T, int NS = 0>
 CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const StreamSet<NZ, double>& St, int k,
                              double gas_od, int kind_rec, const Mat<NZ, double>& T_b, const Mat<NZ, double>& R_b,
                              const double* src_b, double od_b, double B_b, double* g, double (*gs)[3],
@@ -627,7 +628,10 @@ CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const 
       wt[i] = T(St.wt[i]);
       for (int l = 0; l <= nleg; l++) P[i][l] = T(St.P[i][l]);
     }
-    phase_blocks<NZ, T>(nS, nZ, nleg, L.p, P, wt, ff, bb);
+    if constexpr (NS > 0)
+      fixed::phase_blocks<NZ, NS>(L.p, P, wt, ff, bb);
+    else
+      phase_blocks<NZ, T>(nS, nZ, nleg, L.p, P, wt, ff, bb);
     T mx = T(0.0);
     for (int i = 0; i < nZ; i++)
       for (int j = 0; j < nZ; j++) mx = fabs(ff.a[i][j]) > mx ? fabs(ff.a[i][j]) : mx;
@@ -642,6 +646,7 @@ CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const 
     // (PP - PM)(PP + PM), about 1 - ssa, carries FP32's absolute error, and
     // the single-scattering albedo's adjoint loses eps / (1 - ssa): in FP64
     if (fp32 && 1.0 - Ld.ssa < FP32_COALBEDO_MIN) {
+      if constexpr (NS > 0) return LAYER_DEFERRED;
       *in_fp64 = true;
       return 0;
     }
@@ -655,16 +660,24 @@ CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const 
     }
     double gap = 1.0;
     T w_b, tau_b, Bb;
-    const bool ok = ada_layer_adjoint<NZ, T>(nS, nZ, L.ssa, L.od, mu, wt, ff, bb, B, Tb, Rb, sb, &w_b, &tau_b, ffb,
-                                             bbb, &Bb, &gap);
+    bool ok;
+    if constexpr (NS > 0)
+      ok = fixed::ada_layer_adjoint<NZ, NS>(L.ssa, L.od, mu, wt, ff, bb, B, Tb, Rb, sb, &w_b, &tau_b, ffb, bbb, &Bb,
+                                            &gap);
+    else
+      ok = ada_layer_adjoint<NZ, T>(nS, nZ, L.ssa, L.od, mu, wt, ff, bb, B, Tb, Rb, sb, &w_b, &tau_b, ffb, bbb, &Bb,
+                                    &gap);
     if (!ok) {
+      if constexpr (NS > 0) return LAYER_DEFERRED;
       if (!fp32) return -5;
       *in_fp64 = true;   // a failed FP32 factorisation: this layer in FP64
       return 0;
     }
     bool rich = false;
     const double gap_min = fp32 ? FP32_ADJ_GAP_MIN : SENSOR_GAP_MIN;
-    if (gap < gap_min && nZ == nS + 1) {
+    if constexpr (NS > 0) {
+      if (gap < gap_min) return LAYER_DEFERRED;
+    } else if (gap < gap_min && nZ == nS + 1) {
       if (defer) return LAYER_DEFERRED;
       // A quadrature eigenvalue of MOM nearly meets the sensor angle's: the
       // derivatives through the nearly defective eigenbasis lose about
@@ -723,21 +736,24 @@ CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const 
       A.od_b = tau_b;
       A.ssa_b = w_b;
       A.B_b = Bb;
-      phase_blocks_adjoint<NZ, T>(nS, nZ, nleg, L.p, P, wt, ffb, bbb, A.p_b);
+      if constexpr (NS > 0)
+        fixed::phase_blocks_adjoint<NZ, NS>(L.p, P, wt, ffb, bbb, A.p_b);
+      else
+        phase_blocks_adjoint<NZ, T>(nS, nZ, nleg, L.p, P, wt, ffb, bbb, A.p_b);
     }
   }
   if (const int rc = bulk_to_inputs<T>(in, lut, nleg, St.loff, k, in.temperature[k], Ld, A, nsp, g, gs))
     return rc;
   return kind;
 }
-template <int NZ, class T>
+template <int NZ, class T, int NS = 0>
 CRTM_HD int layer_adjoint(const CloudyColumn& in, const CloudLut& lut, const StreamSet<NZ, double>& St, int k,
                           double gas_od, int kind_rec, const Mat<NZ, double>& T_b, const Mat<NZ, double>& R_b,
                           const double* src_b, double od_b, double B_b, double* g, double (*gs)[3], bool defer) {
   bool in_fp64 = false;
-  const int r = layer_adjoint_in<NZ, T>(in, lut, St, k, gas_od, kind_rec, T_b, R_b, src_b, od_b, B_b, g, gs,
-                                        &in_fp64, defer);
-  if constexpr (std::is_same<T, float>::value) {
+  const int r = layer_adjoint_in<NZ, T, NS>(in, lut, St, k, gas_od, kind_rec, T_b, R_b, src_b, od_b, B_b, g, gs,
+                                            &in_fp64, defer);
+  if constexpr (NS == 0 && std::is_same<T, float>::value) {
     // one call site of the FP64 instance for every FP32 fallback
     if (in_fp64) {
       if (defer) return LAYER_DEFERRED;

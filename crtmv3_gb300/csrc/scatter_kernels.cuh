@@ -239,7 +239,7 @@ CRTM_HD int active_species(const CloudyColumn& c, int k, int* sp) {
 
 // One layer's record by one thread, item idx of the chunk (channels fastest).
 // defer: returns true, with nothing written, for a layer that layer_optics defers.
-template <int NZ, class R, class Rec, class C>
+template <int NZ, class R, class Rec, class C, int NS = 0>
 __device__ __forceinline__ bool scatter_layer_item(const ScatterArgs<R>& a, Rec* LBr, long long idx, bool defer) {
   constexpr int NE = layer_record<NZ>();
   const int L = a.L, Kmax = a.Kmax;
@@ -257,11 +257,12 @@ __device__ __forceinline__ bool scatter_layer_item(const ScatterArgs<R>& a, Rec*
     rec[0] = Rec(-rc);
     return false;
   }
+  if (NS > 0 && (S.nS != NS || S.nZ != NS + 1)) return true;
   Mat<NZ, Rec> Tm, Rm;
   Rec src[NZ], od;
   const double gas = double(a.TAU[((size_t)p * Kmax + k) * L + l]);
   double bs = 0.0;
-  const int kind = layer_optics<NZ, Rec, C>(c, a.lut, S, k, C(gas), C(c.temperature[k]), &od, Tm, Rm, src,
+  const int kind = layer_optics<NZ, Rec, C, NS>(c, a.lut, S, k, C(gas), C(c.temperature[k]), &od, Tm, Rm, src,
                                             NoSeed(), nullptr, a.x.sod ? &bs : nullptr, defer);
   if (kind == LAYER_DEFERRED) return true;
   if (kind >= 0) {
@@ -299,7 +300,7 @@ struct ItemLists {
   int* count;        // [n_class + 2]: the classes', then two lists of deferred items
   unsigned* items;   // [n_class + 1][cap] indices in the chunk
   size_t cap;
-  int n_class;       // class 0: nothing scatters; else the number of angles - 1
+  int n_class;       // class 0: nothing scatters; nS - 1: nS quadrature angles and the sensor's; last: others
 };
 
 // Angles of a (profile, channel): stream_set's counts and error codes.
@@ -337,7 +338,7 @@ static __global__ void __launch_bounds__(CLASSIFY_THREADS) scatter_classify_kern
         StreamShape s{0, 1, 0};
         int sp[2 * SC_NC_MAX];
         const bool bad = stream_shape(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, NC, s);
-        cls = bad || active_species(c, k, sp) == 0 ? 0 : s.nZ - 1;
+        cls = bad || active_species(c, k, sp) == 0 ? 0 : (s.nZ > s.nS && s.nS > 1 ? s.nS - 1 : ls.n_class - 1);
       }
     }
   }
@@ -361,18 +362,26 @@ static __global__ void __launch_bounds__(CLASSIFY_THREADS) scatter_classify_kern
   if (cls >= 0) ls.items[(size_t)cls * ls.cap + base[cls] + cnt[wib][cls] + rank] = (unsigned)idx;
 }
 
-// A thread's item of a pass: 0 the classes one after another from the most
-// angles down, each from a CTA's first thread on; 1, 2 the items deferred by
-// the layers' and by the reverse sweep's first pass.
+// Classes with kernels of their own, in which the angle counts are constants:
+// the stream rule's 2 to 4 quadrature angles and the sensor's.  The matrices of
+// a layer are then in registers and no index is computed: a third of the
+// instructions.
+template <int NZ>
+__host__ __device__ constexpr bool fixed_class(int q) { return NZ <= 5 && q >= 1 && q <= 3; }
+// A thread's item of a pass: 0 the classes without a kernel of their own one
+// after another, each from a CTA's first thread on; 1, 2 the items deferred by
+// the layers' and by the reverse sweep's first pass; 3 + q class q.
+template <int NZ>
 __device__ __forceinline__ bool listed_item(const ItemLists& ls, int pass, long long& idx) {
   if (pass > 0) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ls.count[ls.n_class + pass - 1]) return false;
-    idx = ls.items[(size_t)ls.n_class * ls.cap + i];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, q = pass < 3 ? ls.n_class : pass - 3;
+    if (i >= ls.count[pass < 3 ? q + pass - 1 : q]) return false;
+    idx = ls.items[(size_t)q * ls.cap + i];
     return true;
   }
   int c0 = blockIdx.x;
   for (int q = ls.n_class - 1; q >= 0; q--) {
+    if (fixed_class<NZ>(q)) continue;
     const int n = ls.count[q], nb = (n + SCATTER_THREADS - 1) / SCATTER_THREADS;
     if (c0 < nb) {
       const int i = c0 * SCATTER_THREADS + threadIdx.x;
@@ -390,7 +399,7 @@ __device__ __forceinline__ void defer_item(const ItemLists& ls, int pass, long l
 // Threads and CTAs of a pass, for all of a chunk's items however they divide
 // (the counts are on the device; CTAs beyond them end at once).  Deferred
 // items are few and long: one warp a CTA, spread over the SMs.
-inline unsigned list_threads(int pass) { return pass ? 32 : SCATTER_THREADS; }
+inline unsigned list_threads(int pass) { return pass == 1 || pass == 2 ? 32 : SCATTER_THREADS; }
 inline unsigned list_ctas(const ItemLists& ls, int pass) {
   return (unsigned)((ls.cap + list_threads(pass) - 1) / list_threads(pass) + (pass ? 0 : ls.n_class));
 }
@@ -399,8 +408,14 @@ template <int NZ>
 __global__ void __launch_bounds__(SCATTER_THREADS) layers_listed_kernel(ScatterArgs<float> a, float* LBr, ItemLists ls,
                                                                         int pass) {
   long long idx;
-  if (!listed_item(ls, pass, idx)) return;
+  if (!listed_item<NZ>(ls, pass, idx)) return;
   if (scatter_layer_item<NZ, float, float, float>(a, LBr, idx, pass == 0)) defer_item(ls, 1, idx);
+}
+template <int NZ, int NS>
+__global__ void __launch_bounds__(SCATTER_THREADS) layers_fixed_kernel(ScatterArgs<float> a, float* LBr, ItemLists ls) {
+  long long idx;
+  if (!listed_item<NZ>(ls, 2 + NS, idx)) return;
+  if (scatter_layer_item<NZ, float, float, float, NS>(a, LBr, idx, true)) defer_item(ls, 1, idx);
 }
 
 // The forward's further RTSolution components of pair pl (profile p of the
@@ -800,7 +815,7 @@ __global__ void __launch_bounds__(SCATTER_THREADS) scatter_contract_kernel(Scatt
 // layer's inputs in one pass, in the arithmetic C.
 // defer: returns true, with nothing of it written, for a layer that
 // layer_adjoint defers.
-template <int NZ, class R, class C>
+template <int NZ, class R, class C, int NS = 0>
 __device__ __forceinline__ bool scatter_reverse_item(const ScatterArgs<R>& a, long long idx, bool defer) {
   constexpr int NE = layer_record<NZ>();
   const int L = a.L, Kmax = a.Kmax;
@@ -833,6 +848,7 @@ __device__ __forceinline__ bool scatter_reverse_item(const ScatterArgs<R>& a, lo
   }
   StreamSet<NZ, double> S;
   if (stream_set<NZ, double>(c.nleg, c.mu_sensor, c.n_clouds > 0 ? a.lut.nleg : -1, c_gauss, S)) return false;
+  if (NS > 0 && (S.nS != NS || S.nZ != NS + 1)) return true;
   const int nZ = S.nZ;
   Mat<NZ, double> T_b, R_b;
   double src_b[NZ];
@@ -846,7 +862,7 @@ __device__ __forceinline__ bool scatter_reverse_item(const ScatterArgs<R>& a, lo
       src_b[i] = double(rb[(size_t)(2 + 2 * NZ * NZ + i) * L]);
     }
   double g[2], gs[2 * SC_NC_MAX][3];
-  const int kr = layer_adjoint<NZ, C>(c, a.lut, S, k, double(a.TAU[kl]), kind, T_b, R_b, src_b,
+  const int kr = layer_adjoint<NZ, C, NS>(c, a.lut, S, k, double(a.TAU[kl]), kind, T_b, R_b, src_b,
                                       kind == 1 ? 0.0 : od_b, B_b, g, gs, defer);
   if (kr == LAYER_DEFERRED) return true;
   if (kr < 0) {
@@ -880,8 +896,14 @@ template <int NZ>
 __global__ void __launch_bounds__(SCATTER_THREADS, NZ > 5 ? 3 : 1)
     reverse_listed_kernel(ScatterArgs<float> a, ItemLists ls, int pass) {
   long long idx;
-  if (!listed_item(ls, pass, idx)) return;
+  if (!listed_item<NZ>(ls, pass, idx)) return;
   if (scatter_reverse_item<NZ, float, float>(a, idx, pass == 0)) defer_item(ls, 2, idx);
+}
+template <int NZ, int NS>
+__global__ void __launch_bounds__(SCATTER_THREADS) reverse_fixed_kernel(ScatterArgs<float> a, ItemLists ls) {
+  long long idx;
+  if (!listed_item<NZ>(ls, 2 + NS, idx)) return;
+  if (scatter_reverse_item<NZ, float, float, NS>(a, idx, true)) defer_item(ls, 2, idx);
 }
 
 // Species and cloud-fraction Jacobians of one (profile, channel), in place:

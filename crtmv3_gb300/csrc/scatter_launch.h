@@ -24,10 +24,11 @@ int scatter_k_d10f_set_gauss(const GaussTable& g);
 int scatter_soi_d5_set_gauss(const GaussTable& g);
 int scatter_soi_d10_set_gauss(const GaussTable& g);
 int scatter_team_set_gauss(const GaussTable& g);
+int scatter_k_d5x_set_gauss(const GaussTable& g);
 inline int scatter_k_set_gauss(const GaussTable& g) {
   return scatter_k_d5_set_gauss(g) | scatter_k_d10_set_gauss(g) | scatter_k_d5f_set_gauss(g) |
          scatter_k_d10f_set_gauss(g) | scatter_soi_d5_set_gauss(g) | scatter_soi_d10_set_gauss(g) |
-         scatter_team_set_gauss(g);
+         scatter_team_set_gauss(g) | scatter_k_d5x_set_gauss(g);
 }
 
 // FP64 form: layer records (in R) with the layer solver in C
@@ -48,6 +49,9 @@ template <int NZ>
 void launch_layers_listed(const ScatterArgs<float>& a, float* rec, const ItemLists& ls, int pass, cudaStream_t st);
 template <int NZ>
 void launch_reverse_listed(const ScatterArgs<float>& a, const ItemLists& ls, int pass, cudaStream_t st);
+// 5 angles: the classes of constant angle counts (number of kernels launched)
+int launch_layers_fixed(const ScatterArgs<float>& a, float* rec, const ItemLists& ls, cudaStream_t st);
+int launch_reverse_fixed(const ScatterArgs<float>& a, const ItemLists& ls, cudaStream_t st);
 // FP64 form: the ADA profiles' layer contraction (reverse sweep in C)
 template <int NZ, class R, class C>
 void launch_scatter_reverse(const ScatterArgs<R>& a, unsigned grid, cudaStream_t st);

@@ -1081,6 +1081,17 @@ CRTM_HD int species_sums(const CloudyColumn& in, const CloudLut& lut, int nleg, 
   return 0;
 }
 
+// The same for a known angle count: scatter_fixed.cuh.
+namespace fixed {
+template <int NZ, int NS>
+CRTM_HD void phase_blocks(const float* pc, const float (*P)[SC_NLEG_MAX + 1], const float* wt, Mat<NZ, float>& ff,
+                          Mat<NZ, float>& bb);
+template <int NZ, int NS>
+CRTM_HD bool ada_layer_loss(float w, float tau, const float* mu, const float* wt, const Mat<NZ, float>& ff,
+                            const Mat<NZ, float>& bb, float B, Mat<NZ, float>& Um, Mat<NZ, float>& Rm, float* src,
+                            double* gap);
+}  // namespace fixed
+
 // Optics of layer k for the adding method: cloud and aerosol optics summed
 // over the species, combine and delta truncation, and for a scattering layer
 // the phase blocks and the layer's transmission, reflection and source
@@ -1093,8 +1104,10 @@ CRTM_HD int species_sums(const CloudyColumn& in, const CloudLut& lut, int nleg, 
 // defer: an FP32 layer that needs shifted sensor angles or FP64 is not solved;
 // returns LAYER_DEFERRED.  (A run-time choice: the code that solves the other
 // layers is then the same, and so are their bits.)
+// NS > 0: FP32, an ADA layer of NS quadrature angles and the sensor's apart
+// (scatter_fixed.cuh); a layer to be deferred always is.
 constexpr int LAYER_DEFERRED = 2;
-template <int NZ, class T, class S = double, class Seed = NoSeed>
+template <int NZ, class T, class S = double, int NS = 0, class Seed = NoSeed>
 CRTM_HD int layer_optics(const CloudyColumn& in, const CloudLut& lut, const StreamSet<NZ, double>& St, int k,
                          S gas_od, S tk, T* od_out, Mat<NZ, T>& Tm, Mat<NZ, T>& Rm, T* src,
                          Seed seed = Seed(), double* gap = nullptr, double* bs_out = nullptr, bool defer = false) {
@@ -1124,9 +1137,12 @@ CRTM_HD int layer_optics(const CloudyColumn& in, const CloudLut& lut, const Stre
     wt[i] = S(St.wt[i]);
     for (int l = 0; l <= nleg; l++) P[i][l] = S(St.P[i][l]);
   }
-  phase_blocks<NZ, S>(St.nS, St.nZ, nleg, pcs, P, wt, ff, bb);
+  if constexpr (NS > 0)
+    fixed::phase_blocks<NZ, NS>(pcs, P, wt, ff, bb);
+  else
+    phase_blocks<NZ, S>(St.nS, St.nZ, nleg, pcs, P, wt, ff, bb);
   const S B = in.c1 / (exp(in.c2 / (in.b1 + in.b2 * tk)) - 1.0);
-  if (in.soi) {   // SOI: doubling, then the direct beam taken out of the diagonal
+  if (NS == 0 && in.soi) {   // SOI: doubling, then the direct beam taken out of the diagonal
     soi_doubling<NZ, S>(ssa < 0.8 && od < 4.0, St.nS, St.nZ, ssa, od, mu, wt, ff, bb, B, Td, Rd, srcd);
     for (int i = 0; i < St.nZ; i++) Td.a[i][i] -= exp(-od / mu[i]);
   } else {
@@ -1137,9 +1153,14 @@ CRTM_HD int layer_optics(const CloudyColumn& in, const CloudLut& lut, const Stre
     // loss form U = I - T: the record's T = I - U is formed in the record's
     // type, so a layer solved in FP32 keeps its relative precision in FP64 records
     double g32 = 1.0;
-    const bool ok = ada_layer_loss<NZ, S>(St.nS, St.nZ, ssa, od, mu, wt, ff, bb, B, Td, Rd, srcd,
-                                          gap ? gap : &g32);
-    if constexpr (std::is_same<S, float>::value) {
+    bool ok;
+    if constexpr (NS > 0)
+      ok = fixed::ada_layer_loss<NZ, NS>(ssa, od, mu, wt, ff, bb, B, Td, Rd, srcd, &g32);
+    else
+      ok = ada_layer_loss<NZ, S>(St.nS, St.nZ, ssa, od, mu, wt, ff, bb, B, Td, Rd, srcd, gap ? gap : &g32);
+    if constexpr (NS > 0) {
+      if (!ok || g32 < FP32_GAP_MIN) return LAYER_DEFERRED;
+    } else if constexpr (std::is_same<S, float>::value) {
       bool in_fp64 = !ok;
       if (defer && (in_fp64 || ((gap ? *gap : g32) < FP32_GAP_MIN && St.nZ == St.nS + 1))) return LAYER_DEFERRED;
       if (ok && (gap ? *gap : g32) < FP32_GAP_MIN && St.nZ == St.nS + 1) {
