@@ -749,7 +749,8 @@ CRTM_HD int layer_adjoint_in(const CloudyColumn& in, const CloudLut& lut, const 
 template <int NZ, class T, int NS = 0>
 CRTM_HD int layer_adjoint(const CloudyColumn& in, const CloudLut& lut, const StreamSet<NZ, double>& St, int k,
                           double gas_od, int kind_rec, const Mat<NZ, double>& T_b, const Mat<NZ, double>& R_b,
-                          const double* src_b, double od_b, double B_b, double* g, double (*gs)[3], bool defer) {
+                          const double* src_b, double od_b, double B_b, double* g, double (*gs)[3],
+                          bool defer = false) {
   bool in_fp64 = false;
   const int r = layer_adjoint_in<NZ, T, NS>(in, lut, St, k, gas_od, kind_rec, T_b, R_b, src_b, od_b, B_b, g, gs,
                                             &in_fp64, defer);
