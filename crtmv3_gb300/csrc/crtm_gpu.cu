@@ -1670,15 +1670,9 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
         return fail(h, "profile order upload failed");
       dperm = dp;
     }
-    for (int c = 0; c < 3 && rc == CRTM_GPU_SUCCESS; c++) {
-      if (!cnt[c]) continue;
-      crtm_gpu_batch bc = *b;
-      bc.n_profiles = cnt[c];
-      rc = run(&bc, c == 0 && mode == 3 ? 0 : mode, dperm ? nullptr : hc, fixed, c != 0,
-               dperm ? dperm + start[c] : nullptr, c == 2);
-    }
-    // the scattering Jacobians of the clear profiles are zero
-    if (rc == CRTM_GPU_SUCCESS && cnt[0] > 0 && (mode == 1 || mode == 2)) {
+    // the scattering Jacobians of the clear profiles are zero (before the
+    // pipelines: a batch of clear profiles copies its outputs to the host there)
+    if (cnt[0] > 0 && (mode == 1 || mode == 2)) {
       const int NCb = b->max_clouds > 0 ? b->max_clouds : 0, NAb = b->max_aerosols > 0 ? b->max_aerosols : 0;
       const size_t lead = mode == 1 ? (size_t)s.L * b->max_layers : (size_t)b->max_layers;
       double* const outs[7] = {
@@ -1701,6 +1695,13 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
           rc = fail(h, "output clear failed");
         }
       }
+    }
+    for (int c = 0; c < 3 && rc == CRTM_GPU_SUCCESS; c++) {
+      if (!cnt[c]) continue;
+      crtm_gpu_batch bc = *b;
+      bc.n_profiles = cnt[c];
+      rc = run(&bc, c == 0 && mode == 3 ? 0 : mode, dperm ? nullptr : hc, fixed, c != 0,
+               dperm ? dperm + start[c] : nullptr, c == 2);
     }
     if (rc == CRTM_GPU_SUCCESS && dperm && hc && hc->n) rc = copy_chunk(h, hc, 0, P, st);
   }
