@@ -9,9 +9,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcrtm_gb300.so")
 # Translation units, compiled in parallel: the host runtime with the ODPS and
-# forward scattering kernels, and per angle capacity one unit of the
-# scattering K-matrix kernels per arithmetic form and one of the SOI layers'
-# contraction.
+# forward scattering kernels; per angle capacity one unit of the scattering
+# kernels per arithmetic form and one of the SOI layers' contraction; the mixed
+# form's layers of known angle counts and its adding by teams of lanes.
 SOURCES = ["crtm_gpu.cu", "scatter_k_d5.cu", "scatter_k_d10.cu", "scatter_k_d5f.cu", "scatter_k_d10f.cu",
            "scatter_soi_d5.cu", "scatter_soi_d10.cu", "scatter_team.cu", "scatter_k_d5x.cu"]
 HEADERS = ["odps_physics.cuh", "odps_prep.cuh", "odps_kernels.cuh", "optran.cuh", "scatter_physics.cuh",

@@ -11,6 +11,11 @@
 //                          successive orders of interaction (SOI), FP64 in
 //                          every form, then the FP64 Planck inversion.
 //
+// In the mixed form scatter_classify_kernel sorts the chunk's layers into lists,
+// and layers_fixed_kernel / layers_listed_kernel, later reverse_fixed_kernel /
+// reverse_listed_kernel, run them class by class (ItemLists); the K-matrix's
+// adding is adding_front_kernel and adding_team_kernel (scatter_team.cuh).
+//
 // Per-layer results go through HBM with channels fastest:
 // LB[p][k][e][l], e = 0 kind (0 clear, 1 scattering, <0 error), 1 optical
 // depth, then T (NZ*NZ), R (NZ*NZ) and the source (NZ).
@@ -18,7 +23,7 @@
 // K-matrix and adjoint of scattering profiles.  After the first column launch
 // and scatter_layers_kernel (the forward layer records):
 //
-//   scatter_kmatrix_kernel   one thread per (profile, channel): the adding
+//   scatter_kmatrix_kernel   (FP64 form) one thread per (profile, channel): the adding
 //                            from the surface with the level states kept in
 //                            AS, then the adding adjoint from the top down.
 //                            Writes each layer's record adjoints (LBA, FP64:
@@ -28,7 +33,9 @@
 //   scatter_soi_k_kernel     the same for the SOI profiles: the orders of
 //                            interaction with their fields kept (FS), then
 //                            their adjoint from the last order down.
-//   scatter_contract_kernel  one thread per (profile, layer, channel): the
+//   scatter_reverse_kernel   (FP64 form) one thread per (profile, layer,
+//                            channel): the reverse sweep of the ADA layers.
+//   scatter_contract_kernel  (SOI) one thread per (profile, layer, channel): the
 //                            layer optics on derivative numbers (gas optical
 //                            depth, temperature, and each active cloud or
 //                            aerosol's amount and radius), contracted with

@@ -3,9 +3,11 @@
 // the layer solver's (the same); the adding and its adjoint are in R too.
 // A batch with SOI profiles runs in the FP64 form.  Translation units per
 // angle capacity (d5: the stream rule's 2-6 streams, d10: Options%n_Streams
-// up to 16): scatter_k_*.cu (records, adding adjoint, reverse sweep of the ADA
-// layers; the f units for the mixed form) and scatter_soi_*.cu (the SOI
-// layers' derivative-number contraction); they compile in parallel.
+// up to 16): scatter_k_*.cu (FP64 form: records, adding adjoint, reverse sweep of
+// the ADA layers; the f units the mixed form's layers by lists, the x unit those
+// of known angle counts), scatter_team.cu (the mixed form's adding) and
+// scatter_soi_*.cu (the SOI layers' derivative-number contraction); they compile
+// in parallel.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -21,7 +21,7 @@ def _rel(a, b):
 
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("sensor,channels,profiles,layers", [
-    ("mwsynth_c16", 1, 1, (2, 2)), ("mwsynth_c22", 0, 3, (40, 40)), ("mwsynth_c22", 5, 17, (60, 137)),
+    ("mwsynth_c22", 0, 3, (40, 40)), ("mwsynth_c22", 5, 17, (60, 137)),
     ("irsynth_c616", 31, 33, (90, 110)), ("irsynth_c616", 33, 9, (100, 100)), ("irsynth_c616", 65, 8, (127, 129)),
     ("irsynth_c616", 64, 4, (30, 200)), ("irsynth_c616", 0, 2, (199, 200))])
 def test_tile_edges_match_oracle(gpu_lib, coeff_dir, sensor, channels, profiles, layers, precision):
@@ -51,3 +51,10 @@ def test_tile_edges_match_oracle(gpu_lib, coeff_dir, sensor, channels, profiles,
     ad, _ = h.adjoint(atm, sfc, geo, opt, seed)
     kt = np.einsum("pl,plk->pk", seed, km.temperature)
     assert _rel(ad["temperature"], kt) < (1e-5 if precision else 1e-10)
+
+
+def test_too_few_layers_refused(gpu_lib, coeff_dir):
+    """Two layers: more reference layers in a user layer than its band holds."""
+    atm, sfc, geo, opt = sy.clear_sky_workload("mwsynth_c16", 1, np.array([2]), 4001)
+    with pytest.raises(RuntimeError, match="0x8"):
+        gpu_lib.CRTM(["mwsynth_c16"], coeff_dir, 0).forward(atm, sfc, geo, opt)
