@@ -860,6 +860,7 @@ template <int G, class R> constexpr int ad_profiles() { return Tune<G, R>::AD * 
 struct ScatterWork {
   int rec = 0, nz = 0;
   bool soi = false, kstate = false;
+  bool lists = true;     // mixed form: the layers' item lists
   int soi_slots = 0;     // SOI order-field slots of the K-matrix/adjoint
   int slots = 0;         // species Jacobian slots (max_clouds + max_aerosols), 0: none
   bool cf = false;       // cloud-fraction Jacobian
@@ -907,7 +908,7 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
       wk.LBK = (R*)carve(nn * Kmax * (size_t)sw.rec * L * sizeof(R));
     else
       wk.LB = (R*)carve(nn * Kmax * (size_t)sw.rec * L * sizeof(R));
-    if (sizeof(R) == sizeof(float) && !sw.soi)
+    if (sizeof(R) == sizeof(float) && !sw.soi && sw.lists)
       wk.LIST = (unsigned*)carve(nn * Kmax * L * ((sw.nz <= 5 ? 5 : SC_NZ_MAX) + 1) * sizeof(unsigned));
     wk.maxreff = (double*)carve(nn * sizeof(double));
     wk.cover = (double*)carve(nn * sizeof(double));
@@ -1180,7 +1181,7 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
   }
   sw.wind = mode == 2 && sm && sm->ev && ad->wind_speed;
   // chunk size from the workspace budget
-  const size_t per = work_bytes<G, R>(s, 64, Kmax, nv, mode, nullptr, nullptr, sw) / 64 + 1;
+  size_t per = work_bytes<G, R>(s, 64, Kmax, nv, mode, nullptr, nullptr, sw) / 64 + 1;
   int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)P, h->workspace_budget / per));
   if (hc && hc->max_chunk > 0) chunk = std::min(chunk, hc->max_chunk);
   if (scat && sizeof(R) == sizeof(float))   // the scattering item lists hold 32-bit counts and indices
@@ -1189,10 +1190,19 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
   if (!fixed && s.tune_chunk[form] > 0) chunk = std::min(chunk, s.tune_chunk[form]);
   char* ws_base;
   if (fixed) {
+    size_t one = work_bytes<G, R>(s, 1, Kmax, nv, mode, nullptr, nullptr, sw);
+    if (one > fixed->bytes && sizeof(R) == sizeof(float) && scat) {   // without the layers' lists a larger profile fits
+      sw.lists = false;
+      per = work_bytes<G, R>(s, 64, Kmax, nv, mode, nullptr, nullptr, sw) / 64 + 1;
+      one = work_bytes<G, R>(s, 1, Kmax, nv, mode, nullptr, nullptr, sw);
+    }
+    // The limit on a profile of an FP64 K-matrix or adjoint counts the
+    // transmittances and their derivatives that the column keeps in shared
+    // memory, so that it does not depend on where they are kept.
+    if (sizeof(R) == sizeof(double) && (mode == 1 || mode == 2)) one += (sw.rec > 0 ? 1 : 2) * (size_t)Kmax * L * sizeof(R);
     // largest chunk whose workspace fits the fixed scratch
     chunk = (int)std::min<size_t>((size_t)chunk, fixed->bytes / per);
     while (chunk > 1 && work_bytes<G, R>(s, chunk, Kmax, nv, mode, nullptr, nullptr, sw) > fixed->bytes) chunk--;
-    const size_t one = work_bytes<G, R>(s, 1, Kmax, nv, mode, nullptr, nullptr, sw);
     if (chunk < 1 || one > fixed->bytes)
       return fail(h, "one profile of this call needs %zu bytes of scratch (%d channels, max_layers %d, "
                      "%d absorber Jacobians); the static scratch holds %zu bytes",
@@ -1308,14 +1318,16 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
         CK_LAUNCH(h);
         if (listed) {   // mixed form: layers by lists
           if constexpr (mixed) {
-            if (cudaMemsetAsync(lists.count, 0, (lists.n_class + 2) * sizeof(int), st) != cudaSuccess)
-              return fail(h, "cudaMemsetAsync failed");
-            scatter_classify_kernel<<<(unsigned)((nlay + CLASSIFY_THREADS - 1) / CLASSIFY_THREADS), CLASSIFY_THREADS, 0,
-                                      st>>>(sa, lists.n_class, lists);
-            CK_LAUNCH(h);
+            if (sw.lists) {
+              if (cudaMemsetAsync(lists.count, 0, (lists.n_class + 2) * sizeof(int), st) != cudaSuccess)
+                return fail(h, "cudaMemsetAsync failed");
+              scatter_classify_kernel<<<(unsigned)((nlay + CLASSIFY_THREADS - 1) / CLASSIFY_THREADS), CLASSIFY_THREADS,
+                                        0, st>>>(sa, lists.n_class, lists);
+              CK_LAUNCH(h);
+            }
             float* rec = split ? w.LBK : w.LB;
-            if (!nz_max) h->launches += launch_layers_fixed(sa, rec, lists, st);
-            for (int pass = 0; pass <= 1; pass++) {
+            if (sw.lists && !nz_max) h->launches += launch_layers_fixed(sa, rec, lists, st);
+            for (int pass = sw.lists ? 0 : -1; pass <= (sw.lists ? 1 : -1); pass++) {
               if (nz_max)
                 launch_layers_listed<SC_NZ_MAX>(sa, rec, lists, pass, st);
               else
@@ -1360,8 +1372,8 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
         {
           StageScope sc(h, 8, st);
           if constexpr (mixed) {
-            if (!nz_max) h->launches += launch_reverse_fixed(sa, lists, st);
-            for (int pass = 0; pass <= 2; pass += 2) {
+            if (sw.lists && !nz_max) h->launches += launch_reverse_fixed(sa, lists, st);
+            for (int pass = sw.lists ? 0 : -1; pass <= (sw.lists ? 2 : -1); pass += 2) {
               if (nz_max)
                 launch_reverse_listed<SC_NZ_MAX>(sa, lists, pass, st);
               else

@@ -377,9 +377,15 @@ template <int NZ>
 __host__ __device__ constexpr bool fixed_class(int q) { return NZ <= 5 && q >= 1 && q <= 3; }
 // A thread's item of a pass: 0 the classes without a kernel of their own one
 // after another, each from a CTA's first thread on; 1, 2 the items deferred by
-// the layers' and by the reverse sweep's first pass; 3 + q class q.
+// the layers' and by the reverse sweep's first pass; 3 + q class q; -1 (no
+// lists: a static scratch without room for them) the chunk's items in order,
+// nothing deferred.
 template <int NZ>
 __device__ __forceinline__ bool listed_item(const ItemLists& ls, int pass, long long& idx) {
+  if (pass < 0) {
+    idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    return idx < (long long)ls.cap;
+  }
   if (pass > 0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, q = pass < 3 ? ls.n_class : pass - 3;
     if (i >= ls.count[pass < 3 ? q + pass - 1 : q]) return false;

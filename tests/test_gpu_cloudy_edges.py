@@ -59,3 +59,35 @@ def test_results_independent_of_the_batch(gpu_lib, cloud_dir, sensor, streams, c
         assert np.array_equal(rs.radiance, rts.radiance[:, pos])
         for f in FIELDS:
             assert np.array_equal(getattr(ks, f), getattr(km, f)[:, pos]), (n, f)
+
+
+def test_static_scratch_without_room_for_the_lists(gpu_lib, cloud_dir):
+    """The largest profile that the static scratch takes leaves no room for the
+    layers' lists; its layers are then taken in order, with the same bits."""
+    import torch
+    import bench
+    dev = torch.device("cuda")
+    sensor = "irsynth_c2211"
+    h = gpu_lib.CRTM([sensor], cloud_dir, 1)
+    L, stream = h.n_channels[0], torch.cuda.current_stream().cuda_stream
+
+    def call(K, static):
+        atm, sfc, geo, opt = sy.cloudy_workload(sensor, 1, K, 778, wc_scale=50.0)
+        b, keep, t = bench.scatter_device_inputs(torch, h, atm, sfc, geo, opt, dev)
+        out = bench.k_outputs(torch, 1, L, K, atm.n_absorbers, dev)
+        h.k_matrix_device(b, out, None, 0, stream, static_scratch=static)
+        torch.cuda.synchronize()
+        return {f: v.cpu().numpy() for f, v in out.items() if v is not None}
+
+    taken = []
+    for K in range(60, 140):
+        try:
+            taken.append((K, call(K, True)))
+        except RuntimeError as e:
+            assert "static scratch holds" in str(e)
+            break
+    assert 60 < taken[-1][0] < 139
+    for K, got in taken[-3:]:
+        ref = call(K, False)
+        for f in ref:
+            assert np.array_equal(got[f], ref[f]), (K, f)

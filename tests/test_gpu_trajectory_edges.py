@@ -46,7 +46,8 @@ def test_contractions_match_k_matrix(gpu_lib, coeff_dir, channels, layers):
     size = sum(np.abs(x).sum(axis=2) for x in terms)
     assert (np.abs(bt.cpu().numpy() - ref) <= 1e-12 * size).all()
     seed = rng.normal(size=(P, L))
-    out = {"temperature_ad": torch.zeros((P, K), **f64), "water_temperature_ad": torch.zeros((P,), **f64)}
+    out = {"temperature_ad": torch.zeros((P, K), **f64), "absorber_ad": torch.zeros((P, atm.n_absorbers, K), **f64),
+           "water_temperature_ad": torch.zeros((P,), **f64)}
     h.adjoint_apply_device(torch.from_numpy(seed).to(dev), out)
     torch.cuda.synchronize()
     x = km.temperature * seed[:, :, None]
