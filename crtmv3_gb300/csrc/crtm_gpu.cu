@@ -694,6 +694,7 @@ struct crtm_gpu_context {
   std::vector<Sensor> sensors;
   int precision = CRTM_GPU_FP64;
   int device = 0;
+  int smem_max = 48 * 1024;   // shared memory a CTA may take on the device (reserve_smem)
   cudaStream_t stream = nullptr;
   std::string error;
   long long launches = 0;
@@ -962,10 +963,15 @@ BatchView make_view(const crtm_gpu_batch* b) {
   return v;
 }
 
+// Let a kernel (one without static shared memory) take `bytes` of dynamic shared
+// memory.  The limit belongs to the kernel on its device, not to the handle:
+// another thread's call for a smaller batch may come between this one and its
+// launch.  So it is only ever set to the device's maximum, whatever the call needs.
 template <class F>
 int reserve_smem(crtm_gpu_handle h, F kernel, size_t bytes, const char* what) {
-  if (bytes > 48 * 1024 &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+  if (bytes <= 48 * 1024) return CRTM_GPU_SUCCESS;
+  if (bytes > (size_t)h->smem_max ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_max) != cudaSuccess)
     return fail(h, "cannot reserve %zu bytes of shared memory for the %s kernel", bytes, what);
   return CRTM_GPU_SUCCESS;
 }
@@ -2357,6 +2363,7 @@ int crtm_gpu_init_aerosol(const char* coeff_path, int n_sensors, const char* con
   if (cudaGetDevice(&dev) != cudaSuccess) return fail(nullptr, "no CUDA device");
   crtm_gpu_context* h = new crtm_gpu_context();
   h->device = dev;
+  cudaDeviceGetAttribute(&h->smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (const char* e = getenv("CRTM_GPU_WORKSPACE_MB")) h->workspace_budget = (size_t)atoll(e) << 20;
   if (const char* e = getenv("CRTM_GPU_MAP_CHANNELS")) {
     const int v = atoi(e);
