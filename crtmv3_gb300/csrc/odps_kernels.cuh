@@ -1128,11 +1128,11 @@ __global__ void __launch_bounds__(128) column_kernel(ColumnArgs<R> a) {
 //    the layer adjoints, the reference levels' path adjoints).
 //
 //    Bound: FP64 issue (an exponential is some 25 instructions of 64 clocks
-//    each per scheduler), so two exponentials a layer, reciprocals instead of
-//    divisions, and the transmittance above a layer from the recursion.  A
+//    each per scheduler), so two exponentials and two divisions a layer, and the
+//    transmittance above a layer from the recursion.  A
 //    thread per (profile, channel) kept one of an SM's four schedulers busy for
-//    a single 22-channel profile (246 us, now 58) and evaluated the exponentials
-//    once per pass (K-matrix columns of 250 x 616: 5.6 ms, now 4.3).  In the
+//    a single 22-channel profile (246 us, now 57) and evaluated the exponentials
+//    once per pass (K-matrix columns of 250 x 616: 5.6 ms, now 4.4).  In the
 //    mixed form the recursions' latency weighs more than the exponentials: the
 //    tile took 7.3 ms for 1000 x 2211 K-matrix columns against 3.4 ms, so it
 //    keeps the thread per pair.
@@ -1235,6 +1235,7 @@ __global__ void __launch_bounds__(COL_THREADS) column_tile_kernel(ColumnArgs<R> 
       sP[c] = R(0);
       spec[c] = R(a.sp.c1[l]); spec[cw + c] = R(a.sp.c2[l]);
       spec[2 * cw + c] = R(a.sp.b1[l]); spec[3 * cw + c] = R(a.sp.b2[l]);
+      if (adj) { spec[5 * cw + c] = R(a.sp.b2[l] / a.sp.c2[l]); spec[6 * cw + c] = R(1.0 / a.sp.c1[l]); }
     }
   }
   const double* sc = a.pv.scal + (size_t)p * PREP_SCAL;
@@ -1284,16 +1285,16 @@ __global__ void __launch_bounds__(COL_THREADS) column_tile_kernel(ColumnArgs<R> 
       sTau[ku * CS + c] = tau;
       if ((a.mode == 3 || a.pass == 1) && chan) a.TAU[cs + (size_t)ku * L] = tau;
       if (a.mode == 3 || (a.pass == 1 && scat_p)) continue;
-      // (reciprocals: an FP64 division costs as much as ten multiplications)
-      const R rte = R(1) / (b1 + b2 * tus[ku]);
-      const R ee = exp(c2 * rte);
-      const R rem1 = R(1) / (ee - R(1));
+      // The exponent rounds once (a reciprocal of te, multiplied, would round
+      // twice: rms error of B 3.0e-16 instead of 2.2e-16 at 700 cm-1, 1.03e-15
+      // instead of 7.2e-16 at 2500), and dB/dT = (b2 / c2) q^2 (B + B^2 / c1) needs
+      // no division of its own (rms 1.7e-16 and 6.4e-16; with a third division of
+      // c1 c2 b2 e^q by (te (e^q - 1))^2 2.6e-16 and 7.3e-16).
+      const R q = c2 / (b1 + b2 * tus[ku]);
+      const R B = c1 / (exp(q) - R(1));
       sT[ku * CS + c] = exp(-tau * inv_u);
-      sB[ku * CS + c] = c1 * rem1;
-      if (adj) {
-        const R rden = rte * rem1;
-        sD[ku * CS + c] = c1 * c2 * b2 * ee * rden * rden;
-      }
+      sB[ku * CS + c] = B;
+      if (adj) sD[ku * CS + c] = spec[5 * cw + c] * (q * q) * (B + B * (B * spec[6 * cw + c]));
     }
   }
   __syncthreads();
