@@ -818,7 +818,7 @@ struct Work {
   PrepView<R> pv;
   R* OD;            // [n][K][L]
   R* TAU, *DTOP;    // [n][Kmax][L] (FP64 form: TAU of batches with clouds or aerosols)
-  R* FIN;           // FP64 form: [n][4][L] column_tile_kernel -> column_finish_kernel
+  R* FIN;           // FP64 form: [n][4][L] column_tile_kernel -> column_finish_kernel (K-matrix, adjoint: in RA)
   R* PT;            // [n][Kmax][L]
   R* SC;            // [n][L]
   double* TSK;      // adjoint: [n][L]
@@ -902,7 +902,7 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
   wk.pv = pv;
   wk.OD = (R*)carve(nn * K * L * sizeof(R));
   constexpr bool tile = sizeof(R) == sizeof(double);   // column_tile_kernel
-  if (tile) wk.FIN = (R*)carve(nn * 4 * L * sizeof(R));
+  if (tile && mode == 0) wk.FIN = (R*)carve(nn * 4 * L * sizeof(R));
   if (sw.rec > 0 || (adj && !tile)) wk.TAU = (R*)carve(nn * Kmax * L * sizeof(R));
   if (sw.rec > 0) {
     if (sw.kstate)
@@ -935,7 +935,8 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
     if (!tile) wk.DTOP = (R*)carve(nn * Kmax * L * sizeof(R));
     wk.PT = (R*)carve(nn * Kmax * L * sizeof(R));
     wk.SC = (R*)carve(nn * L * sizeof(R));
-    wk.RA = (R*)carve(nn * nv * K * L * sizeof(R));
+    wk.RA = (R*)carve(nn * std::max(nv * K, 4) * L * sizeof(R));
+    if (tile) wk.FIN = wk.RA;   // free until absorb_ad_kernel
   }
   if (mode == 2 && sw.wind) wk.WS = (double*)carve(nn * L * sizeof(double));
   if (mode == 2) {
@@ -947,6 +948,23 @@ size_t work_bytes(const Sensor& s, int n, int Kmax, int nv, int mode, Work<R>* w
   wk.idx_map = (int*)carve((MAX_ABS + SC_NZ_MAX + 2) * sizeof(int));
   if (w) *w = wk;
   return off;
+}
+
+// What a profile counts as against a fixed scratch beyond what it takes: the
+// limit of the entry point (which calls it takes and which it refuses) does not
+// move with where the kernels keep their values.  It is that of an FP64 K-matrix or
+// adjoint with the column's transmittances and downwelling radiances in scratch
+// (column_tile_kernel keeps them, or all but the transmittances of batches with
+// clouds or aerosols, in shared memory) and the predictor partials of 2 profiles a
+// warp, group 3 of 4 (now one).  Never negative: a profile that is taken fits.
+template <int G, class R>
+size_t fixed_scratch_reserve(const Sensor& s, int Kmax, int mode, const ScatterWork& sw) {
+  if (sizeof(R) != sizeof(double) || (mode != 1 && mode != 2)) return 0;
+  constexpr int counted = G == 3 ? 4 : 2;
+  static_assert(counted >= Tune<G, double>::AD, "the limit counts what the kernels take");
+  const size_t partials = (size_t)AD_WARPS * s.K * DLayout<G>::NX * sizeof(R);
+  return align_up(counted * partials) - align_up(Tune<G, R>::AD * partials) +
+         (sw.rec > 0 ? 1 : 2) * align_up((size_t)Kmax * s.L * sizeof(R));
 }
 
 BatchView make_view(const crtm_gpu_batch* b) {
@@ -1202,15 +1220,12 @@ int run_pipeline(crtm_gpu_handle h, const Sensor& s, const crtm_gpu_batch* b, in
       per = work_bytes<G, R>(s, 64, Kmax, nv, mode, nullptr, nullptr, sw) / 64 + 1;
       one = work_bytes<G, R>(s, 1, Kmax, nv, mode, nullptr, nullptr, sw);
     }
-    // The limit on a profile of an FP64 K-matrix or adjoint counts the
-    // transmittances and their derivatives that the column keeps in shared
-    // memory, so that it does not depend on where they are kept.
-    if (sizeof(R) == sizeof(double) && (mode == 1 || mode == 2)) one += (sw.rec > 0 ? 1 : 2) * (size_t)Kmax * L * sizeof(R);
+    one += fixed_scratch_reserve<G, R>(s, Kmax, mode, sw);
     // largest chunk whose workspace fits the fixed scratch
     chunk = (int)std::min<size_t>((size_t)chunk, fixed->bytes / per);
     while (chunk > 1 && work_bytes<G, R>(s, chunk, Kmax, nv, mode, nullptr, nullptr, sw) > fixed->bytes) chunk--;
     if (chunk < 1 || one > fixed->bytes)
-      return fail(h, "one profile of this call needs %zu bytes of scratch (%d channels, max_layers %d, "
+      return fail(h, "one profile of this call counts as %zu bytes of scratch (%d channels, max_layers %d, "
                      "%d absorber Jacobians); the static scratch holds %zu bytes",
                   one, L, Kmax, nv - 1, fixed->bytes);
     ws_base = fixed->base;
