@@ -1703,9 +1703,9 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
         return fail(h, "profile order upload failed");
       dperm = dp;
     }
-    // the scattering Jacobians of the clear profiles are zero (before the
-    // pipelines: a batch of clear profiles copies its outputs to the host there)
-    if (cnt[0] > 0 && (mode == 1 || mode == 2)) {
+    // the scattering Jacobians of the clear profiles are zero
+    auto zero_clear = [&]() -> int {
+      if (cnt[0] == 0 || (mode != 1 && mode != 2)) return CRTM_GPU_SUCCESS;
       const int NCb = b->max_clouds > 0 ? b->max_clouds : 0, NAb = b->max_aerosols > 0 ? b->max_aerosols : 0;
       const size_t lead = mode == 1 ? (size_t)s.L * b->max_layers : (size_t)b->max_layers;
       double* const outs[7] = {
@@ -1725,10 +1725,16 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
           zero_profile_rows_kernel<<<(unsigned)((nel + 255) / 256), 256, 0, st>>>(outs[i], dperm, cnt[0], rows[i]);
           CK_LAUNCH(h);
         } else if (cudaMemsetAsync(outs[i], 0, (size_t)P * rows[i] * sizeof(double), st) != cudaSuccess) {
-          rc = fail(h, "output clear failed");
+          return fail(h, "output clear failed");
         }
       }
-    }
+      return CRTM_GPU_SUCCESS;
+    };
+    // A host batch of one bucket copies its outputs from the pipeline, chunk by
+    // chunk: its zeros come first.  Other calls write them last, so that a call
+    // that the pipeline refuses has launched nothing and touched no output.
+    const bool zero_first = !dperm && hc;
+    if (zero_first) rc = zero_clear();
     for (int c = 0; c < 3 && rc == CRTM_GPU_SUCCESS; c++) {
       if (!cnt[c]) continue;
       crtm_gpu_batch bc = *b;
@@ -1736,6 +1742,7 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
       rc = run(&bc, c == 0 && mode == 3 ? 0 : mode, dperm ? nullptr : hc, fixed, c != 0,
                dperm ? dperm + start[c] : nullptr, c == 2);
     }
+    if (rc == CRTM_GPU_SUCCESS && !zero_first) rc = zero_clear();
     if (rc == CRTM_GPU_SUCCESS && dperm && hc && hc->n) rc = copy_chunk(h, hc, 0, P, st);
   }
   mark_done(h, st);

@@ -1,4 +1,5 @@
-"""What crtm_gpu_k_matrix_device_static takes and refuses, at the limit.
+"""What crtm_gpu_k_matrix_device_static takes and refuses, at the limit, and that
+a refused call launches nothing and leaves its outputs as they were.
 
 The FP64 limit counts a profile's K-matrix intermediates as the entry point was
 released with: predictors, partials, bands, reference and user layer arrays,
@@ -32,10 +33,11 @@ def wide(gpu_lib, tmp_path_factory):
     tc = sy.generate_odps(3, L, 5, SID, co.INFRARED_SENSOR, max_predictors_per_channel=1)
     co.write_odps(os.path.join(d, f"{SID}.TauCoeff.bin"), tc)
     co.write_spccoeff(os.path.join(d, f"{SID}.SpcCoeff.bin"), sy.generate_spccoeff(SID, co.INFRARED_SENSOR, L, 6))
+    sy.write_cloud_files(d)
     return gpu_lib.CRTM([SID], d, 0)
 
 
-def _call(h, atm, sfc, geo, static):
+def _call(h, atm, sfc, geo, static, species=0):
     import torch
     import bench
     dev = torch.device("cuda")
@@ -43,6 +45,9 @@ def _call(h, atm, sfc, geo, static):
     opt = sy.OptionsBatch(emissivity=sy.emissivity_for(co.INFRARED_SENSOR, P, L, 10))
     b, keep, t = bench.scatter_device_inputs(torch, h, atm, sfc, geo, opt, dev)
     out = {k: v.fill_(-7) for k, v in bench.k_outputs(torch, P, L, Km, J, dev).items()}
+    if species:
+        for f in ("cloud_water_content_k", "cloud_effective_radius_k"):
+            out[f] = torch.full((P, L, species, Km), -7.0, dtype=torch.float64, device=dev)
     try:
         h.k_matrix_device(b, out, None, 0, torch.cuda.current_stream().cuda_stream, static_scratch=static)
         return out, None
@@ -66,3 +71,43 @@ def test_limit(wide):
     out, err = _call(wide, atm, sfc, geo, True)
     assert "static scratch holds" in err and f" {_counted(131, 7)} bytes" in err
     assert wide.launch_count() == launches
+
+
+@pytest.mark.parametrize("clear", [(0, 1), (0,)])
+def test_refused_call_leaves_outputs_alone(wide, clear):
+    """Cloud arrays with clear profiles beside a cloudy one, and clear ones alone."""
+    atm, sfc, geo = sy.generate_profiles(2, 200, sy.absorber_set(1), 9)
+    sy.add_clouds(atm, (co.WATER_CLOUD, co.ICE_CLOUD), 12)
+    atm.n_clouds[list(clear)] = 0
+    launches = wide.launch_count()
+    out, err = _call(wide, atm, sfc, geo, True, species=atm.cloud_type.shape[1])
+    assert "static scratch holds" in err
+    assert wide.launch_count() == launches
+    for f, v in out.items():
+        assert bool((v == -7).all()), f
+
+
+@pytest.mark.parametrize("clear", [(0, 1), (0,)])
+def test_clear_profiles_scattering_jacobians_are_zero(gpu_lib, coeff_dir, clear):
+    """Of device and of host calls, into buffers that hold something else."""
+    import torch
+    import bench
+    sy.write_cloud_files(coeff_dir)
+    sensor, dev = "mwsynth_c16", torch.device("cuda")
+    atm, sfc, geo, opt = sy.cloudy_workload(sensor, 2, 60, 31, wc_scale=50.0)
+    atm.n_clouds[list(clear)] = 0
+    for precision in (0, 1):
+        h = gpu_lib.CRTM([sensor], coeff_dir, precision)
+        km, _ = h.k_matrix(atm, sfc, geo, opt)
+        b, keep, t = bench.scatter_device_inputs(torch, h, atm, sfc, geo, opt, dev)
+        out = bench.k_outputs(torch, 2, 16, 60, atm.n_absorbers, dev)
+        NC = atm.cloud_type.shape[1]
+        for f in ("cloud_water_content", "cloud_effective_radius"):
+            out[f + "_k"] = torch.full((2, 16, NC, 60), -7.0, dtype=torch.float64, device=dev)
+        h.k_matrix_device(b, out, None, 0, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        for f in ("cloud_water_content", "cloud_effective_radius"):
+            got = out[f + "_k"].cpu().numpy()
+            assert np.array_equal(got, getattr(km, f)), f
+            for p in range(2):
+                assert (got[p] == 0.0).all() == (p in clear), (f, p)
