@@ -240,7 +240,7 @@ CRTM_HD bool ada_layer_loss(float w, float tau, const float* mu, const float* wt
   mat_mul(nZ, Rn, A, V);
   for (int i = 0; i < nZ; i++)
     for (int j = 0; j < nZ; j++) { Um.a[i][j] = X.a[i][j]; Rm.a[i][j] = V.a[i][j]; }
-  // source (1 - row sum of float + R) B over the quadrature columns (and T's
+  // source (1 - row sum of T + R) B over the quadrature columns (and T's
   // diagonal on the sensor row) = (row sum of U - row sum of R) B
   for (int i = 0; i < nZ; i++) {
     float a = 0.0f;
@@ -290,7 +290,7 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
   // U = (Q D + Gp W) GA^-1 = I - T,  R = (Gp D + Gm D P e) GA^-1.  Every
   // term of U and R is O(tau) for a thin layer, and so is every adjoint that
   // reaches the eigen-decomposition below: the FP32 form keeps its relative
-  // accuracy where the plain form float = Tt GA^-1 loses it to cancellation.
+  // accuracy where the plain form T = Tt GA^-1 loses it to cancellation.
   const float s = w < float(MAX_ALBEDO) ? w : float(MAX_ALBEDO);
   Mat<NZ, float> E, iX, Gp, Gm, iGm, P, W, iGA, Um, Rm, T1, T2;
   float lam[NZ], ev[NZ], ex[NZ], dx[NZ], buf[NZ];
@@ -352,8 +352,8 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
     }
   }
   *B_b = bsum;
-  // U = Un GA^-1, R = Rn GA^-1:  Un_b = U_b GA^-T, Rn_b = R_b GA^-float (row by
-  // row in place), then GA_b = -(U^float Un_b + R^float Rn_b) into iGA
+  // U = Un GA^-1, R = Rn GA^-1:  Un_b = U_b GA^-T, Rn_b = R_b GA^-T (row by
+  // row in place), then GA_b = -(U^T Un_b + R^T Rn_b) into iGA
   for (int i = 0; i < n; i++) {
     for (int j = 0; j < n; j++) {
       float v = 0.0f;
@@ -380,7 +380,7 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
   float dx_b[NZ], ex_b[NZ];
   for (int j = 0; j < n; j++) { dx_b[j] = 0.0f; ex_b[j] = 0.0f; }
   // Un = Q D + Gp W, GA = Q + Gp W:  Q_b = Un_b D + GA_b;  dx_b_j += sum_i Un_b_ij Q_ij;
-  //   with S = Un_b + GA_b (T1):  W_b = Gp^float S;  Gp_b = S W^T
+  //   with S = Un_b + GA_b (T1):  W_b = Gp^T S;  Gp_b = S W^T
   for (int i = 0; i < n; i++)
     for (int j = 0; j < n; j++) {
       float v = 0.0f;
@@ -394,8 +394,8 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
   mat_mul_nt(n, T1, W, Gpb);
   Mat<NZ, float>& Gmb = T1;    // S is dead
   // Rn = Gp D + Gm D P e:  Gp_b += Rn_b D;  dx_b_j += sum_i Rn_b_ij Gp_ij;
-  //   ex_b_j += sum_i Rn_b_ij (Gm D P)_ij;  with Z = Rn_b e:  Gm_b = Z P^float D,
-  //   dx_b_k += sum_i Gm_ik (Z P^T)_ik;  P_b = D Gm^float Z (column by column into T2)
+  //   ex_b_j += sum_i Rn_b_ij (Gm D P)_ij;  with Z = Rn_b e:  Gm_b = Z P^T D,
+  //   dx_b_k += sum_i Gm_ik (Z P^T)_ik;  P_b = D Gm^T Z (column by column into T2)
   for (int i = 0; i < n; i++)
     for (int j = 0; j < n; j++) {
       const float rb = T2.a[i][j];
@@ -421,7 +421,7 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
     for (int k = 0; k < n; k++) T2.a[k][j] = buf[k];
   }
   Mat<NZ, float>& Pb = T2;
-  // Q = Gm - Gp P:  Gm_b += Q_b;  Gp_b -= Q_b P^T;  P_b -= Gp^float Q_b
+  // Q = Gm - Gp P:  Gm_b += Q_b;  Gp_b -= Q_b P^T;  P_b -= Gp^T Q_b
   for (int i = 0; i < n; i++)
     for (int j = 0; j < n; j++) {
       float a = 0.0f, b = 0.0f;
@@ -442,7 +442,7 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
       ex_b[j] = add_prod(ex_b[j], wb * dx[i], pij);
       dx_b[j] += prod(wb, pij);
     }
-  // P = Gm^-1 Gp:  K = Gm^-float P_b;  Gp_b += K;  Gm_b -= K P^T
+  // P = Gm^-1 Gp:  K = Gm^-T P_b;  Gp_b += K;  Gm_b -= K P^T
   Mat<NZ, float>& Kt = Um;   // Q_b is dead
   mat_mul_tn(n, iGm, Pb, Kt);
   for (int i = 0; i < n; i++)
@@ -461,7 +461,7 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
       Eb.a[i][j] = prod(0.5f, p + q);
       EFb.a[i][j] = prod(0.5f, p - q);
     }
-  // EF = iX E diag(ev):  iX_b = EF_b (E diag(ev))^T;  EV_b = iX^float EF_b;
+  // EF = iX E diag(ev):  iX_b = EF_b (E diag(ev))^T;  EV_b = iX^T EF_b;
   //   E_b += EV_b diag(ev);  ev_b_j = sum_i EV_b_ij E_ij
   Mat<NZ, float>& iXb = Um;   // K is dead
   Mat<NZ, float>& EVb = Rm;   // W_b is dead
@@ -487,10 +487,10 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
     lam_b[j] = lam[j] > 0.0f ? 0.5f * ev_b / ev[j] : 0.0f;
   }
   *tau_b = tb;
-  // X = PP - PM inverted:  X_b = -iX^float iX_b iX^float  (in P; W is scratch)
+  // X = PP - PM inverted:  X_b = -iX^T iX_b iX^T  (in P; W is scratch)
   Mat<NZ, float>& Xb = P;
   inverse_adjoint(n, iX, iXb, Xb, W);
-  // HH = E diag(lam) E^-1:  HH_b = E^-float (diag(lam_b) + F o (E^float E_b)) E^T,
+  // HH = E diag(lam) E^-1:  HH_b = E^-T (diag(lam_b) + F o (E^T E_b)) E^T,
   // F_ij = 1 / (lam_j - lam_i) off the diagonal
   Mat<NZ, float>& Ei = Gp;    // Gp, Gm, iGm are dead
   Mat<NZ, float>& Mx = Gm;
@@ -501,10 +501,10 @@ CRTM_HD bool ada_layer_adjoint(float w, float tau, const float* mu, const float*
     for (int j = 0; j < n; j++)
       Mx.a[i][j] = (i == j) ? lam_b[i] : Mx.a[i][j] / (lam[j] - lam[i]);
   Mat<NZ, float>& HHb = Rm;   // EV_b is dead
-  mat_mul_tn(n, Ei, Mx, T2);   // E^-float M  (P_b is dead)
-  mat_mul_nt(n, T2, E, HHb);   // (E^-float M) E^T
+  mat_mul_tn(n, Ei, Mx, T2);   // E^-T M  (P_b is dead)
+  mat_mul_nt(n, T2, E, HHb);   // (E^-T M) E^T
   // HH = X Y with X = PP - PM, Y = PP + PM (rebuilt from the phase blocks):
-  //   X_b += HH_b Y^T;  Y_b = X^float HH_b
+  //   X_b += HH_b Y^T;  Y_b = X^T HH_b
   Mat<NZ, float>& X = iGm;
   Mat<NZ, float>& Y = W;
   for (int i = 0; i < n; i++) {
