@@ -480,7 +480,7 @@ def pipe_peaks(torch, dev):
 
 
 # Operations of one scattering layer's MOM work in the cloudy K-matrix's
-# layer reverse sweep (scatter_reverse_kernel: phase blocks, the loss-form MOM
+# layer reverse sweep (reverse_fixed_kernel, reverse_listed_kernel: phase blocks, the loss-form MOM
 # forward and its reverse sweep, the phase blocks' adjoint) by its angle
 # count nZ, counted by running the kernel's header code on an
 # operation-counting number type (tests/harness/flop_count.cpp; every +, -,
@@ -661,8 +661,9 @@ def run_scattering(args, torch, dev, rank, world, dist):
             pipe = "fp32"   # the mixed form's adding and reverse sweep run in FP32
             roofline = {"bound": pipe, "achieved": ach, "peak": pk[pipe], "unit": "TFLOP/s",
                         "frac": ach / pk[pipe], "traffic": None,
-                        "kernel": ("scatter_kmatrix_kernel (adding + adjoint)" if dom == "scatter_adding" else
-                                   "scatter_reverse_kernel (MOM forward + reverse sweep per scattering layer)"),
+                        "kernel": ("adding_team_kernel (adding + adjoint)" if dom == "scatter_adding" else
+                                   "reverse_fixed_kernel, reverse_listed_kernel (MOM forward + reverse sweep per "
+                                   "scattering layer)"),
                         "algorithmic_flops_per_step": fl,
                         "flop_count": ("38 nZ^3 per scattering layer" if dom == "scatter_adding" else
                                        "REVERSE_LAYER_OPS[nZ] per scattering layer, counted on an "

@@ -1572,10 +1572,12 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
   if (cudaSetDevice(h->device) != cudaSuccess) return fail(h, "cudaSetDevice failed");
   const Sensor& s = h->sensors[sensor];
   const bool scat = b->max_clouds > 0 || b->max_aerosols > 0;
-  // The mixed form runs the gas optics and the scattering layer solver in
-  // FP32 and the adding in FP64.  The K-matrix and adjoint of a batch with
-  // SOI profiles (Options%RT_Algorithm_Id given) run in the FP64 form: the SOI
-  // layers' doubling and its derivative-number contraction are FP64 only.
+  // The mixed form runs the gas optics and the scattering layer solver in FP32,
+  // the forward's adding in FP64 on FP32 records, and the K-matrix's and adjoint's
+  // adding in FP32 with its inverses in FP64 where the layers couple strongly.
+  // The K-matrix and adjoint of a batch with SOI profiles (Options%RT_Algorithm_Id
+  // given) run in the FP64 form: the SOI layers' doubling and its
+  // derivative-number contraction are FP64 only.
   const bool fp64 = h->precision == CRTM_GPU_FP64 ||
                     (scat && (mode == 1 || mode == 2) && b->rt_algorithm_id != nullptr);
   if (scat) {

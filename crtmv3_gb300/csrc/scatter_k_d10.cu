@@ -20,8 +20,7 @@ void launch_scatter_layers_k(const ScatterArgs<R>& a, unsigned grid, cudaStream_
 template <int NZ, class R>
 void launch_scatter_kmatrix(const ScatterArgs<R>& a, dim3 grid, cudaStream_t st, bool soi) {
   scatter_kmatrix_kernel<NZ, R><<<grid, SCATTER_THREADS, 0, st>>>(a);
-  if constexpr (std::is_same<R, double>::value)
-    if (soi) scatter_soi_k_kernel<NZ><<<grid, SCATTER_THREADS, 0, st>>>(a);
+  if (soi) scatter_soi_k_kernel<NZ><<<grid, SCATTER_THREADS, 0, st>>>(a);
 }
 
 template <int NZ, class R, class C>
