@@ -1128,11 +1128,11 @@ __global__ void __launch_bounds__(128) column_kernel(ColumnArgs<R> a) {
 //    the layer adjoints, the reference levels' path adjoints).
 //
 //    Bound: FP64 issue (an exponential is some 25 instructions of 64 clocks
-//    each per scheduler), so two exponentials and two divisions a layer, and the
-//    transmittance above a layer from the recursion.  A
+//    each per scheduler), so two exponentials and two quotients (a reciprocal each) a
+//    layer, and the transmittance above a layer from the recursion.  A
 //    thread per (profile, channel) kept one of an SM's four schedulers busy for
-//    a single 22-channel profile (246 us, now 57) and evaluated the exponentials
-//    once per pass (K-matrix columns of 250 x 616: 5.6 ms, now 4.4).  In the
+//    a single 22-channel profile (246 us, now 53) and evaluated the exponentials
+//    once per pass (K-matrix columns of 250 x 616: 5.6 ms, now 4.3).  In the
 //    mixed form the recursions' latency weighs more than the exponentials: the
 //    tile took 7.3 ms for 1000 x 2211 K-matrix columns against 3.4 ms, so it
 //    keeps the thread per pair.
@@ -1165,6 +1165,16 @@ inline int column_cshift(int K, int Kmax, int L, int n, bool full) {
   while (c > 2 && column_tile_smem_bytes<R>(K, Kmax, c, full) > 112 * 1024) c--;
   while (c > 2 && (long long)n * ((L + (1 << c) - 1) >> c) < 152 * 2) c--;
   return c;
+}
+
+// a / b from b's reciprocal and one correction by the quotient's residual
+// (P. Markstein, IBM J. Res. Dev. 34 (1990) 111): the division's value but for
+// rare last places, in two multiply-adds more than the product (forward of
+// 1500 x 22 channels 1.77 ms with divisions, 1.68 with this).  Where the
+// correction has no finite value (b zero or infinite), the product stands.
+__device__ __forceinline__ double quotient(double a, double b) {
+  const double r = 1.0 / b, q = a * r, c = fma(fma(-q, b, a), r, q);
+  return (__double2hiint(c) & 0x7ff00000) == 0x7ff00000 ? q : c;
 }
 
 // EXT: the call asks for further RTSolution components (a.x); without them
@@ -1290,8 +1300,8 @@ __global__ void __launch_bounds__(COL_THREADS) column_tile_kernel(ColumnArgs<R> 
       // instead of 7.2e-16 at 2500), and dB/dT = (b2 / c2) q^2 (B + B^2 / c1) needs
       // no division of its own (rms 1.7e-16 and 6.4e-16; with a third division of
       // c1 c2 b2 e^q by (te (e^q - 1))^2 2.6e-16 and 7.3e-16).
-      const R q = c2 / (b1 + b2 * tus[ku]);
-      const R B = c1 / (exp(q) - R(1));
+      const R q = quotient(c2, b1 + b2 * tus[ku]);
+      const R B = quotient(c1, exp(q) - R(1));
       sT[ku * CS + c] = exp(-tau * inv_u);
       sB[ku * CS + c] = B;
       if (adj) sD[ku * CS + c] = spec[5 * cw + c] * (q * q) * (B + B * (B * spec[6 * cw + c]));
