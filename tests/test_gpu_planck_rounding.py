@@ -50,3 +50,17 @@ def test_layer_planck_radiance_rounds_its_exponent_once(gpu_lib, tmp_path, call)
     r = 1.0 / -np.expm1(-x[ok])
     bound = np.sqrt(np.mean(r ** 2 * (np.spacing(x[ok]) ** 2 / 12.0 + 4.0 * U ** 2) + 2.0 / 3.0 * U ** 2))
     assert np.sqrt(np.mean(err ** 2)) <= bound
+
+
+def test_overflowing_exponential_is_zero_radiance(gpu_lib, coeff_dir):
+    """A layer so cold that e^x has no finite value emits nothing: c1 / inf = 0."""
+    sensor, P = "irsynth_c2211", 3
+    spc = co.read_spccoeff(os.path.join(coeff_dir, f"{sensor}.SpcCoeff.bin"))
+    atm, sfc, geo, opt = sy.clear_sky_workload(sensor, P, 40, 43)
+    atm.temperature[:, 0] = [1.0, 2.0, 250.0]
+    x = spc.planck_c2[None] / (spc.band_c1[None] + spc.band_c2[None] * atm.temperature[:, :1])
+    assert (x > 711.0).any(axis=1).tolist() == [True, True, False]
+    rts = gpu_lib.CRTM([sensor], coeff_dir, 0).forward(atm, sfc, geo, opt, components=True)
+    got = rts.upwelling_overcast_radiance[:, :, 0]
+    assert (got[x > 711.0] == 0.0).all() and (got[x < 700.0] > 0.0).all()
+    assert np.isfinite(rts.radiance).all() and np.isfinite(rts.brightness_temperature).all()
