@@ -1734,7 +1734,7 @@ int dispatch(crtm_gpu_handle h, int sensor, const crtm_gpu_batch* b, int mode, c
     };
     // A host batch of one bucket copies its outputs from the pipeline, chunk by
     // chunk: its zeros come first.  Other calls write them last, so that a call
-    // that the pipeline refuses has launched nothing and touched no output.
+    // whose first pipeline refuses it has launched nothing and touched no output.
     const bool zero_first = !dperm && hc;
     if (zero_first) rc = zero_clear();
     for (int c = 0; c < 3 && rc == CRTM_GPU_SUCCESS; c++) {
